@@ -144,7 +144,7 @@ def build_ref_gpu():
 
 def build(ref=True):
     built = [build_oracle()]
-    if ref and os.path.isdir(REF):
+    if ref and os.path.isdir(os.path.join(REF, "cuda", "velo")):  # the folder may be there and empty
         os.makedirs(OUT, exist_ok=True)
         built.append(build_ref_x86())
         built.append(build_ref_checker())
