@@ -7,12 +7,13 @@
 //   * seeding: the phi windows of every h1 come precomputed from fill_candidates (in the
 //     pruned mode the scorer has cleared the windows of pruned seeds, and forwarding skips
 //     candidates without the extension-keep bit when that pruning is on);
-//     the h1 candidates of a step are compacted into a shared list, their
-//     (h1, h0) pairs are flattened over the lanes, and each h1 keeps its best triplet in a
-//     shared 64-bit key (scatter bits, h0 offset, h2 offset) reduced with atomicMin. The
-//     winner is the minimal scatter, first in (h0, h2) order; an atomicMax twin with the
-//     scatter bits inverted finds the last candidate of equal scatter, so exact ties (which
-//     the reference resolves by thread scheduling) are flagged;
+//     the h1 candidates of a step are compacted into a shared list and searched in three
+//     passes (seed_flush below): their (h1, h0) pairs flattened over the lanes, which keeps the
+//     pairs inside the slope cut; a lane per kept pair, which marks the h2 of its window near the
+//     straight line; and the marked triplets over the lanes, which get the reference's test.
+//     Each h1 keeps its best triplet in a shared 64-bit key (scatter bits, h0 offset, h2
+//     offset): the winner is the minimal scatter, first in (h0, h2) order, and exact ties
+//     (which the reference resolves by thread scheduling) are flagged;
 //   * hit_used is a bitmask in shared memory; appends to the ring buffers go in lane order
 //     through ballots, so the result does not depend on scheduling.
 #pragma once
@@ -35,11 +36,17 @@ __device__ __forceinline__ uint32_t ballot_rank(bool pred, uint32_t& total)
   return __popc(b & ((1u << lane_id()) - 1u));
 }
 
-// Scatter of the triplet (h0, h1, h2) and whether it passes the seeding cuts
-// (TrackSeeding.cu:137-152).
-__device__ __forceinline__ bool seed_scatter(const float4 h0, const float4 h1, const float4 h2, float& scatter)
+// Slope cut of the doublet (h0, h1) (TrackSeeding.cu:137-152).
+__device__ __forceinline__ bool seed_slope(const float4 h0, const float4 h1)
 {
   const float dmax = kMaxSlope * (h0.z - h1.z);
+  return fabsf(h1.x - h0.x) < dmax && fabsf(h1.y - h0.y) < dmax;
+}
+
+// Scatter of the triplet (h0, h1, h2) and whether it passes the seeding cuts beyond the
+// doublet's slope (TrackSeeding.cu:137-152).
+__device__ __forceinline__ bool seed_triplet(const float4 h0, const float4 h1, const float4 h2, float& scatter)
+{
   const float scatterDenom2 = 1.f / ((h2.z - h1.z) * (h2.z - h1.z));
   const float z2_tz = (h2.z - h0.z) / (h1.z - h0.z);
   const float x = h0.x + (h1.x - h0.x) * z2_tz;
@@ -48,8 +55,12 @@ __device__ __forceinline__ bool seed_scatter(const float4 h0, const float4 h1, c
   const float dy = y - h2.y;
   const float scatterNum = (dx * dx) + (dy * dy);
   scatter = scatterNum * scatterDenom2;
-  return fabsf(h1.x - h0.x) < dmax && fabsf(h1.y - h0.y) < dmax && fabsf(dx) < kTolerance && fabsf(dy) < kTolerance &&
-         scatter < kMaxScatterSeeding;
+  return fabsf(dx) < kTolerance && fabsf(dy) < kTolerance && scatter < kMaxScatterSeeding;
+}
+
+__device__ __forceinline__ bool seed_scatter(const float4 h0, const float4 h1, const float4 h2, float& scatter)
+{
+  return seed_slope(h0, h1) && seed_triplet(h0, h1, h2, scatter);
 }
 
 // Forwarding fit of one candidate (TrackForwarding.cu:12-35).
@@ -142,16 +153,183 @@ __device__ __forceinline__ float weak_chi2(const float4* H, const uint16_t* h)
   return ch / nDoF;
 }
 
+constexpr uint32_t kPairQueue = 64;  // doublets waiting for a full round of 32
+
 struct SeedSlots {
   uint16_t h1[kSeedChunk];
   uint16_t f0[kSeedChunk];
   uint16_t f2[kSeedChunk];
-  uint16_t l2[kSeedChunk];
-  uint16_t np[kSeedChunk];
-  uint32_t pair_start[kSeedChunk];
-  unsigned long long best[kSeedChunk];
-  unsigned long long last[kSeedChunk];
+  uint16_t n2[kSeedChunk];
+  uint32_t pair_start[kSeedChunk];    // number of h0 of each candidate, then its exclusive scan
+  unsigned long long best[kSeedChunk];  // scatter bits << 32 | h0 offset << 16 | h2 offset
+  uint32_t tie[kSeedChunk];           // smallest scatter that two triplets share
+  uint32_t pair[kPairQueue];          // candidate << 16 | h0 offset in its window
+  uint32_t triplet[32];               // lane of its pair << 16 | h2 offset
 };
+
+// Exclusive scan of v[0 .. n) in place by one warp; returns the total.
+__device__ __forceinline__ uint32_t warp_scan_in_place(uint32_t* v, uint32_t n)
+{
+  const uint32_t lane = lane_id();
+  uint32_t total = 0;
+  for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const uint32_t x = k < n ? v[k] : 0;
+    uint32_t incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= static_cast<uint32_t>(o)) incl += t;
+    }
+    if (k < n) v[k] = total + incl - x;
+    total += __shfl_sync(0xFFFFFFFFu, incl, 31);
+  }
+  __syncwarp();
+  return total;
+}
+
+// Segment of position p0 + lane, for p0 = 0, 32, 64, ... in turn: start[0 .. n) are the
+// segments' first positions (no segment is empty), `lo` the segment of position p0 - 1 (0 at
+// first; advanced here). The segments starting inside the 32 positions are lo + 1 .. lo + 32,
+// so one shared load, an OR across the warp and a popcount replace a binary search.
+__device__ __forceinline__ uint32_t warp_segment(const uint32_t* start, uint32_t n, uint32_t p0, uint32_t& lo)
+{
+  const uint32_t lane = lane_id();
+  uint32_t head = 0;
+  if (lo + 1 + lane < n) {
+    const uint32_t s = start[lo + 1 + lane] - p0;
+    if (s < 32u) head = 1u << s;
+  }
+  const uint32_t heads = __reduce_or_sync(0xFFFFFFFFu, head);
+  const uint32_t k = lo + __popc(heads & (0xFFFFFFFFu >> (31 - lane)));
+  lo = __shfl_sync(0xFFFFFFFFu, k, 31);
+  return k;
+}
+
+// The triplets of the first n (<= 32) queued pairs, by one warp: a lane per pair marks the h2
+// of its window near the straight line through h0 and h1, and the marked ones, packed over the
+// lanes, get the reference's test (TrackSeeding.cu:137-175) and compete for their candidate's
+// key.
+//
+// The marking is a superset of the reference's cut: its prediction and the reference's differ
+// by the rounding of a quotient, a product and a sum, at most 7.2e-7 (|x| + |x0|); the box is
+// widened by 1e-5 of both and by 1e-4 mm (a NaN marks). So the loop over a window, whose length
+// the longest window of the 32 pairs sets, holds no division and no branch.
+__device__ __forceinline__ void seed_round(SeedSlots& sl, uint32_t n, const float4* H, const uint32_t* used)
+{
+  const uint32_t lane = lane_id();
+  uint32_t n2 = 0, f2 = 0;
+  float x0 = 0.f, y0 = 0.f, z0 = 0.f, tx = 0.f, ty = 0.f, tol0 = 0.f;
+  if (lane < n) {
+    const uint32_t pk = sl.pair[lane], k = pk >> 16;
+    const float4 h0 = H[sl.f0[k] + (pk & 0xFFFFu)];
+    const float4 h1 = H[sl.h1[k]];
+    f2 = sl.f2[k];
+    n2 = sl.n2[k];
+    x0 = h0.x;
+    y0 = h0.y;
+    z0 = h0.z;
+    const float inv = __fdividef(1.f, h1.z - h0.z);
+    tx = (h1.x - h0.x) * inv;
+    ty = (h1.y - h0.y) * inv;
+    tol0 = kTolerance + 1e-4f + 1e-5f * fmaxf(fabsf(x0), fabsf(y0));
+  }
+  const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, n2);
+  for (uint32_t c0 = 0; c0 < longest; c0 += 32) {
+    uint32_t marks = 0;
+    const uint32_t m = n2 > c0 ? min(n2 - c0, 32u) : 0u;
+    const float4* W = H + f2 + c0;
+#pragma unroll 2
+    for (uint32_t j = 0; j < m; ++j) {
+      const float4 h2 = W[j];
+      const float dz = h2.z - z0;
+      const float x = x0 + tx * dz;
+      const float y = y0 + ty * dz;
+      const float d = fmaxf(fabsf(x - h2.x), fabsf(y - h2.y));
+      const float tol = tol0 + 1e-5f * fmaxf(fabsf(x), fabsf(y));
+      if (!(d >= tol)) marks |= 1u << j;
+    }
+    const uint32_t cnt = __popc(marks);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= static_cast<uint32_t>(o)) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    uint32_t pos = incl - cnt;
+    for (uint32_t w0 = 0; w0 < total; w0 += 32) {
+      while (marks && pos < w0 + 32) {
+        sl.triplet[pos - w0] = (lane << 16) | (c0 + __ffs(marks) - 1);
+        marks &= marks - 1;
+        ++pos;
+      }
+      __syncwarp();
+      if (w0 + lane < total) {
+        const uint32_t t = sl.triplet[lane], pk = sl.pair[t >> 16], k = pk >> 16;
+        const uint32_t h2rel = t & 0xFFFFu, h2i = sl.f2[k] + h2rel;
+        if (!test_used(used, h2i)) {
+          float scatter;
+          if (seed_triplet(H[sl.f0[k] + (pk & 0xFFFFu)], H[sl.h1[k]], H[h2i], scatter)) {
+            const uint32_t sb = __float_as_uint(scatter);
+            const unsigned long long key = (static_cast<unsigned long long>(sb) << 32) | (pk << 16) | h2rel;
+            // once the smallest scatter has come, every equal one meets it here
+            const unsigned long long old = atomicMin(&sl.best[k], key);
+            if (static_cast<uint32_t>(old >> 32) == sb) atomicMin(&sl.tie[k], sb);
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// Seeding of the nc candidates queued in `sl` by one warp (TrackSeeding.cu:90-183): leaves
+// each candidate's best triplet in sl.best.
+//
+// Bound by instruction issue and by the latency of the hit records. A lane per (h1, h0) pair
+// that tested every h2 of its window kept 17.8 lanes busy (the longest window of 32 pairs sets
+// the loop) at about 35 instructions a step; here the pairs outside the slope cut (42% of the
+// triplets) leave first and the step of the window loop is 15 instructions. Search of 65,536
+// events at nu ~ U(2,20) 15.16 -> 13.80 ms (1.41 -> 1.23 G warp instructions per 8,192 events),
+// of 3,000 events at nu = 15 with noise 8.31 -> 6.04 ms. Flattening the triplets too kept 24
+// lanes busy and was slower (15.5 and 9.2 ms): locating a triplet costs more than its test.
+__device__ __forceinline__ void seed_flush(SeedSlots& sl, uint32_t nc, const float4* H, const uint32_t* used)
+{
+  const uint32_t lane = lane_id();
+  __syncwarp();
+  const uint32_t total_pairs = warp_scan_in_place(sl.pair_start, nc);
+  uint32_t n_queued = 0;
+  uint32_t k_lo = 0;  // candidate of the last pair seen
+  for (uint32_t p0 = 0; p0 < total_pairs; p0 += 32) {
+    const uint32_t p = p0 + lane;
+    const uint32_t k = warp_segment(sl.pair_start, nc, p0, k_lo);
+    bool pair = false;
+    uint32_t h0rel = 0;
+    if (p < total_pairs) {
+      h0rel = p - sl.pair_start[k];
+      const uint32_t h0i = sl.f0[k] + h0rel;
+      if (!test_used(used, h0i)) pair = seed_slope(H[h0i], H[sl.h1[k]]);
+    }
+    uint32_t n_new;
+    const uint32_t rank = ballot_rank(pair, n_new);
+    if (pair) sl.pair[n_queued + rank] = (k << 16) | h0rel;
+    n_queued += n_new;
+    const bool last = p0 + 32 >= total_pairs;
+    while (n_queued >= 32 || (last && n_queued > 0)) {
+      __syncwarp();
+      const uint32_t n = min(n_queued, 32u);
+      seed_round(sl, n, H, used);
+      // the pairs beyond the round move to the front
+      n_queued -= n;
+      uint32_t v = 0;
+      if (lane < n_queued) v = sl.pair[32 + lane];
+      __syncwarp();
+      if (lane < n_queued) sl.pair[lane] = v;
+    }
+  }
+  __syncwarp();
+}
 
 // Forwarding reads the phi of its two target modules from shared memory; the staging
 // area reuses the seeding slots (the two phases never overlap).
@@ -279,69 +457,9 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
     // module's first ones. The two modules' seeds are independent (seeding marks no hit
     // used), and winners are appended in queue order, the order of a pass per module.
     uint32_t nc = 0;  // candidates queued
-    // (b)-(d) on the queued candidates
     auto flush = [&]() {
-      __syncwarp();
-      // (b) exclusive scan of the h0 counts
-      uint32_t total_pairs = 0;
-      for (uint32_t k0 = 0; k0 < nc; k0 += 32) {
-        const uint32_t k = k0 + lane;
-        const uint32_t v = k < nc ? sl.np[k] : 0;
-        uint32_t incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-          if (lane >= static_cast<uint32_t>(o)) incl += t;
-        }
-        if (k < nc) sl.pair_start[k] = total_pairs + incl - v;
-        total_pairs += __shfl_sync(0xFFFFFFFFu, incl, 31);
-      }
-      __syncwarp();
-      // (c) (h1, h0) pairs over the lanes, each scanning its h2 window. Every candidate
-      // has at least one pair (a non-empty window ends past its first hit), so the
-      // candidates starting inside a group of 32 pairs are k_lo + 1 .. k_lo + 32 and
-      // each lane's candidate is k_lo plus the starts at or before it (one shared
-      // load, an OR across the warp and a popcount instead of a binary search).
-      uint32_t k_lo = 0;  // candidate of pair p0
-      for (uint32_t p0 = 0; p0 < total_pairs; p0 += 32) {
-        const uint32_t p = p0 + lane;
-        uint32_t head = 0;
-        if (k_lo + 1 + lane < nc) {
-          const uint32_t s = sl.pair_start[k_lo + 1 + lane];
-          if (s >= p0 && s <= p0 + 31) head = 1u << (s - p0);
-        }
-        const uint32_t heads = __reduce_or_sync(0xFFFFFFFFu, head);
-        const uint32_t k = k_lo + __popc(heads & (0xFFFFFFFFu >> (31 - lane)));
-        k_lo = __shfl_sync(0xFFFFFFFFu, k, 31);
-        if (p < total_pairs) {
-          const uint32_t h0rel = p - sl.pair_start[k];
-          const uint32_t h0i = sl.f0[k] + h0rel;
-          if (!test_used(used, h0i)) {
-            const float4 h0 = H[h0i];
-            const float4 h1 = H[sl.h1[k]];
-            const uint32_t f2 = sl.f2[k], l2 = sl.l2[k];
-            unsigned long long best = ~0ull, last = 0ull;
-            for (uint32_t h2i = f2; h2i < l2; ++h2i) {
-              if (test_used(used, h2i)) continue;
-              float scatter;
-              if (seed_scatter(h0, h1, H[h2i], scatter)) {
-                const uint32_t idx = (h0rel << 16) | (h2i - f2);
-                const uint32_t sb = __float_as_uint(scatter);
-                const unsigned long long key = (static_cast<unsigned long long>(sb) << 32) | idx;
-                const unsigned long long key_last = (static_cast<unsigned long long>(~sb) << 32) | idx;
-                best = min(best, key);
-                last = max(last, key_last);
-              }
-            }
-            if (best != ~0ull) {
-              atomicMin(&sl.best[k], best);
-              atomicMax(&sl.last[k], last);
-            }
-          }
-        }
-      }
-      __syncwarp();
-      // (d) winners, appended in candidate order (TrackSeeding.cu:185-195)
+      seed_flush(sl, nc, H, used);
+      // winners, appended in candidate order (TrackSeeding.cu:185-195)
       for (uint32_t k0 = 0; k0 < nc; k0 += 32) {
         const uint32_t k = k0 + lane;
         const bool win = k < nc && sl.best[k] != ~0ull;
@@ -349,7 +467,7 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
         const uint32_t rank = ballot_rank(win, nwin);
         if (win) {
           const unsigned long long key = sl.best[k];
-          if ((key & 0xFFFFFFFFull) != (sl.last[k] & 0xFFFFFFFFull)) flags |= kStatusSeedTie;
+          if (static_cast<uint32_t>(key >> 32) == sl.tie[k]) flags |= kStatusSeedTie;
           const uint32_t tp = (tracklet_ptr + rank) % kTrackletRing;
           tracklets[3 * tp] = static_cast<uint16_t>(sl.f0[k] + ((key >> 16) & 0xFFFFu));
           tracklets[3 * tp + 1] = sl.h1[k];
@@ -410,11 +528,11 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
           const uint32_t f0 = w.x & 0xFFFFu, l0 = w.x >> 16, f2 = w.y & 0xFFFFu, l2 = w.y >> 16;
           sl.h1[k] = static_cast<uint16_t>(h1);
           sl.f0[k] = static_cast<uint16_t>(f0);
-          sl.np[k] = static_cast<uint16_t>(l0 - f0);
           sl.f2[k] = static_cast<uint16_t>(f2);
-          sl.l2[k] = static_cast<uint16_t>(l2);
+          sl.n2[k] = static_cast<uint16_t>(l2 - f2);
+          sl.pair_start[k] = l0 - f0;
           sl.best[k] = ~0ull;
-          sl.last[k] = 0ull;
+          sl.tie[k] = 0xFFFFFFFFu;
         }
         nc += cnt;
       }
