@@ -292,4 +292,32 @@ __device__ __forceinline__ void phi_window(const float* phis, uint32_t start, ui
   }
 }
 
+// phi_window over n (> 0) sorted phi in shared memory, n the same for every lane of the warp:
+// the partition points of the reference's two searches by halving steps without a branch, and
+// its "found" flag from the elements beside the first one. The flag says whether an element
+// that the search probes lies within the margin. The one it ends on is probed; when that one
+// lies outside, so does every other (|value - e| grows away from value, rounded too), except
+// where value - margin and value - e round to different sides of the cut at the window's lower
+// edge: there the reference's own search decides.
+__device__ __forceinline__ void phi_window_flat(const float* a, uint32_t n, float value, float margin, int& first,
+                                                int& last)
+{
+  const float lo = value - margin, hi = value + margin;
+  // il: the first element not below lo, or the last element; ih: the same for hi
+  uint32_t il = 0, ih = 0;
+  for (uint32_t len = n; len > 1;) {
+    const uint32_t half = len >> 1;
+    if (lo > a[il + half - 1]) il += half;
+    if (hi > a[ih + half - 1]) ih += half;
+    len -= half;
+  }
+  const float el = a[il];
+  bool found = fabsf(value - el) < margin;
+  if (!found && !(lo > el) && (el < value || (il > 0 && fabsf(value - a[il - 1]) < margin)))
+    found = window_first(a, n, value, margin) != -1;
+  const int s = static_cast<int>(ih - il) + (fabsf(value - a[ih]) < margin ? 1 : 0);
+  first = found ? static_cast<int>(il) : -1;
+  last = found ? static_cast<int>(il) + max(s, 1) : -1;
+}
+
 }  // namespace velo

@@ -331,9 +331,9 @@ __device__ __forceinline__ void seed_flush(SeedSlots& sl, uint32_t nc, const flo
   __syncwarp();
 }
 
-// Forwarding reads the phi of its two target modules from shared memory; the staging
-// area reuses the seeding slots (the two phases never overlap).
-constexpr uint32_t kFwdStage = sizeof(SeedSlots) / (2 * sizeof(float));
+// Forwarding reads the phi of its two target modules from shared memory, one after the other
+// in a staging area that reuses the seeding slots (the two phases never overlap).
+constexpr uint32_t kFwdStage = sizeof(SeedSlots) / sizeof(float);
 
 struct SearchWarpShared {
   uint32_t used[kEventHitCap / 32];
@@ -341,7 +341,7 @@ struct SearchWarpShared {
   uint32_t mnum[kModules];
   union {
     SeedSlots seed;
-    float fphi[2][kFwdStage];
+    float fphi[kFwdStage];
   } u;
 };
 
@@ -369,11 +369,60 @@ __device__ __forceinline__ void forward_window_staged(const float4* H, const flo
     flags |= kStatusEmptyModuleRead;
     return;
   }
-  phi_window(sphi, 0, mnum, phi, kForwardPhiTolerance, first, last);
+  phi_window_flat(sphi, mnum, phi, kForwardPhiTolerance, first, last);
   if (first != -1) {
     first += static_cast<int>(mstart);
     last += static_cast<int>(mstart);
   }
+}
+
+// Best forwarding fit of one track (direction tx, ty of its last hits h0 -> h1) over the n
+// candidates of its two windows, first in order on equal fits (TrackForwarding.cu:41-110):
+// candidate j is hit odd + j below n_odd and even + j from there on. FLT_MAX: none fits.
+//
+// Two passes over up to 32 candidates: a loop without a division or a branch marks the ones
+// near the prediction - a superset of the reference's box, widened by more than the rounding of
+// its sum (a NaN marks) - and the marked ones, one in eight, get the reference's fit. The first
+// loop's length is set by the longest windows among the warp's tracks (42% of its lanes are
+// busy), so its step decides: 15 instructions against 40 with the fit inside. With the
+// branch-free window searches, search of 65,536 events at nu ~ U(2,20) 13.80 -> 13.35 ms.
+__device__ __forceinline__ float forward_best(const float4* H, const uint8_t* KE, const float4 h0, const float4 h1,
+                                              float tx, float ty, int odd, int n_odd, int even, int n,
+                                              uint16_t& best_h2)
+{
+  float best_fit = 3.402823466e+38f;
+  const float tol0 = kTolerance + 1e-4f + 1e-5f * fmaxf(fabsf(h0.x), fabsf(h0.y));
+  for (int c0 = 0; c0 < n; c0 += 32) {
+    const int m = min(n - c0, 32);
+    uint32_t marks = 0;
+#pragma unroll 2
+    for (int j = 0; j < m; ++j) {
+      const float4 h2 = H[c0 + j + (c0 + j < n_odd ? odd : even)];
+      const float dz = h2.z - h0.z;
+      const float x = h0.x + tx * dz;
+      const float y = h0.y + ty * dz;
+      const float d = fmaxf(fabsf(x - h2.x), fabsf(y - h2.y));
+      const float tol = tol0 + 1e-5f * fmaxf(fabsf(x), fabsf(y));
+      if (!(d >= tol)) marks |= 1u << j;
+    }
+    while (marks) {
+      const int j = c0 + __ffs(marks) - 1;
+      marks &= marks - 1;
+      const int h2i = j + (j < n_odd ? odd : even);
+      if (KE && !(KE[h2i] & 2u)) continue;
+      const float4 h2 = H[h2i];
+      const float dz = h2.z - h0.z;
+      const float predx = tx * dz;
+      const float predy = ty * dz;
+      const float scatterDenom2 = 1.f / ((h2.z - h1.z) * (h2.z - h1.z));
+      const float fit = forward_fit(h0.x, h0.y, h2.x, h2.y, predx, predy, scatterDenom2);
+      if (fit < best_fit) {
+        best_fit = fit;
+        best_h2 = static_cast<uint16_t>(h2i);
+      }
+    }
+  }
+  return best_fit;
 }
 
 // Per-event scratch of the warp search: the reference's Velo::TrackHits slots and the rings
@@ -550,15 +599,14 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
     const uint32_t mo = first - 4, me = first - 5;
     const uint32_t mos = mstart[mo], mon = mnum[mo], mes = mstart[me], men = mnum[me];
     const float moz = c_module_z[mo], mez = c_module_z[me];
-    // stage the phi of both target modules (their binary searches then stay in shared
-    // memory); a module above the staging size is searched in global memory
-    const float* sphi_o = mon <= kFwdStage ? sw.u.fphi[0] : nullptr;
-    const float* sphi_e = men <= kFwdStage ? sw.u.fphi[1] : nullptr;
-    if (diff > 0) {
-      if (sphi_o)
-        for (uint32_t i = lane; i < mon; i += 32) sw.u.fphi[0][i] = H[mos + i].w;
-      if (sphi_e)
-        for (uint32_t i = lane; i < men; i += 32) sw.u.fphi[1][i] = H[mes + i].w;
+    // stage the phi of both target modules (their searches then stay in shared memory); a pair
+    // of modules above the staging size is searched in global memory
+    const bool fits = mon + men <= kFwdStage;
+    const float* sphi_o = fits ? sw.u.fphi : nullptr;
+    const float* sphi_e = fits ? sw.u.fphi + mon : nullptr;
+    if (diff > 0 && fits) {
+      for (uint32_t i = lane; i < mon; i += 32) sw.u.fphi[i] = H[mos + i].w;
+      for (uint32_t i = lane; i < men; i += 32) sw.u.fphi[mon + i] = H[mes + i].w;
     }
     __syncwarp();
     for (uint32_t i0 = 0; i0 < diff; i0 += 32) {
@@ -591,25 +639,11 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
         const float tyn = (h1.y - h0.y);
         const float tx = txn * td;
         const float ty = tyn * td;
-        float best_fit = 3.402823466e+38f;
         int of, ol, ef, el;
         forward_window_staged(H, sphi_o, mos, mon, moz, tx, ty, h0.x, h0.y, h0.z, true, of, ol, flags);
         forward_window_staged(H, sphi_e, mes, men, mez, tx, ty, h0.x, h0.y, h0.z, false, ef, el, flags);
         const int n_odd = ol - of, n_even = el - ef;
-        for (int j = 0; j < n_odd + n_even; ++j) {
-          const int h2i = j < n_odd ? of + j : ef + j - n_odd;
-          if (KE && !(KE[h2i] & 2u)) continue;
-          const float4 h2 = H[h2i];
-          const float dz = h2.z - h0.z;
-          const float predx = tx * dz;
-          const float predy = ty * dz;
-          const float scatterDenom2 = 1.f / ((h2.z - h1.z) * (h2.z - h1.z));
-          const float fit = forward_fit(h0.x, h0.y, h2.x, h2.y, predx, predy, scatterDenom2);
-          if (fit < best_fit) {
-            best_fit = fit;
-            best_h2 = static_cast<uint16_t>(h2i);
-          }
-        }
+        const float best_fit = forward_best(H, KE, h0, h1, tx, ty, of, n_odd, ef - n_odd, n_odd + n_even, best_h2);
         // a track holds at most one hit per module pair: 26 hits (VeloDefinitions.cuh:26)
         if (best_fit != 3.402823466e+38f && nhit < kMaxTrackSize) action = 1;
         else if (skipped < kMaxSkippedModules) action = 2;
