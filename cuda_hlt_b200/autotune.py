@@ -1,7 +1,7 @@
 """Autotuner of the launch shapes, by timing stages on a sample batch:
 
-* the search mapping: the cluster count above which an event runs the block-per-event search
-  instead of the warp-per-event one (hit-count buckets);
+* the search mapping: the cluster count above which an event takes a block in the search
+  whatever the batch (hit-count buckets);
 * the decode block size: 4 or 8 warps per event (the tile of SuperPixels one block sorts and
   clusters at a time)."""
 import numpy as np

@@ -194,7 +194,8 @@ class VeloChain:
         _check(self.lib.velo_set_mlp(self.ctx, C.byref(weights), C.sizeof(weights)), "velo_set_mlp")
 
     def set_block_threshold(self, clusters):
-        """Events above `clusters` clusters use the block-per-event search, others the warp one."""
+        """Events above `clusters` clusters always take a block in the search (>= 16384: none but
+        those the mapping's own rule gives one)."""
         _check(self.lib.velo_set_block_threshold(self.ctx, int(clusters)), "velo_set_block_threshold")
 
     def set_decode_warps(self, warps):

@@ -19,7 +19,6 @@
 #include "velo_fill.cuh"
 #include "velo_order.cuh"
 #include "velo_search.cuh"
-#include "velo_search_block.cuh"
 #include "velo_consolidate.cuh"
 #include "velo_pv.cuh"
 #include "velo_gec.cuh"
@@ -77,7 +76,7 @@ struct VeloCtx {
   uint32_t *d_atomics = nullptr, *d_track_hit_number = nullptr, *d_event_hit_offset = nullptr;
   char *d_track_hits_out = nullptr, *d_states = nullptr, *d_kalman = nullptr;
   uint32_t* d_queue = nullptr;
-  uint32_t *d_warp_events = nullptr, *d_block_events = nullptr, *d_event_order = nullptr;
+  uint32_t* d_event_order = nullptr;
   uint32_t block_threshold = 0;  // clusters above which an event takes the block search
   // beamline PV stage (velo_set_pv)
   bool pv = false;
@@ -115,7 +114,7 @@ struct VeloCtx {
   int ev_current = -1;
   int decode_warps = 8;
   int search_wpb = 4;
-  uint32_t decode_blocks = 0, search_blocks = 0, search_block_blocks = 0, fill_blocks = 0,
+  uint32_t decode_blocks = 0, search_blocks = 0, fill_blocks = 0,
            feature_blocks = 0, score_blocks = 0;
   // CUDA graphs per (batch-size bucket, stream, global event cut on or off): the kernels read
   // the run's inputs from d_run, so a graph serves every batch of its bucket; at most
@@ -167,7 +166,7 @@ void free_all(VeloCtx* c)
                   c->d_event_hits, c->d_status, c->d_track_n, c->d_track_hits, c->d_tracklets, c->d_weak, c->d_ttf,
                   c->d_event_tracks, c->d_event_track_hits, c->d_atomics, c->d_track_hit_number,
                   c->d_event_hit_offset, c->d_track_hits_out, c->d_states, c->d_kalman, c->d_queue,
-                  c->d_warp_events, c->d_block_events, c->d_event_order, c->d_pv_tracks, c->d_pv_vertices,
+                  c->d_event_order, c->d_pv_tracks, c->d_pv_vertices,
                   c->d_pv_count, c->d_pv_npeaks, c->d_pv_zpeaks, c->d_gec_counts, c->d_event_list,
                   c->d_n_selected, c->d_gec_flags, c->d_gec_ut, c->d_gec_scifi, c->d_gec_ut_offsets,
                   c->d_gec_scifi_offsets};
@@ -235,10 +234,9 @@ ChainPointers pointers(VeloCtx* c, uint32_t n_grid)
   P.max_track_hits_total = c->cfg.max_track_hits;
   P.hit_capacity = c->hit_capacity;
   P.queue = c->d_queue;
-  P.warp_events = c->d_warp_events;
   P.event_order = c->d_event_order;
-  P.block_events = c->d_block_events;
   P.block_threshold = c->block_threshold;
+  P.search_warps = c->search_blocks * kSearchWarps;
   P.mlp = c->mlp;
   if (c->mode == VELO_MODE_LABELS) {
     P.mlp = MlpDevice{};
@@ -352,21 +350,12 @@ int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaS
   VCK(cudaGetLastError());
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][2], s, capturing));
   {
-    // both mappings: each kernel drains its own event list (routed by the decode kernel)
-    if (c->block_threshold > 0) {
-      order_events_kernel<<<1, kOrderThreads, 0, s>>>(P);
-      VCK(cudaGetLastError());
-      const uint32_t blocks = std::min<uint32_t>((n + 3) / 4, c->search_blocks);
-      search_kernel<4><<<blocks, 128, 0, s>>>(P);
-      VCK(cudaGetLastError());
-      c->launches += 2;
-    }
-    if (c->block_threshold < kEventHitCap) {
-      const uint32_t blocks = std::min<uint32_t>(n, c->search_block_blocks);
-      search_block_kernel<<<blocks, kBlockThreads, kStageCap * sizeof(float4), s>>>(P);
-      VCK(cudaGetLastError());
-      ++c->launches;
-    }
+    order_events_kernel<<<1, kOrderThreads, 0, s>>>(P);
+    VCK(cudaGetLastError());
+    // at least a block for each event that might take one
+    search_kernel<kSearchWarps><<<std::min<uint32_t>(n, c->search_blocks), kSearchWarps * 32, 0, s>>>(P);
+    VCK(cudaGetLastError());
+    c->launches += 2;
   }
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][3], s, capturing));
   event_scan_kernel<<<1, 1024, 0, s>>>(P);
@@ -401,7 +390,7 @@ void size_decode_grid(VeloCtx* c)
 void size_search_grid(VeloCtx* c)
 {
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_kernel<4>, 128, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_kernel<kSearchWarps>, kSearchWarps * 32, 0);
   c->search_blocks = static_cast<uint32_t>(std::max(1, occ) * c->sm_count);
 }
 
@@ -541,8 +530,6 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   ok &= dalloc(c->d_gec_ut_offsets, static_cast<size_t>(N) + 1) == cudaSuccess;
   ok &= dalloc(c->d_gec_scifi_offsets, static_cast<size_t>(N) + 1) == cudaSuccess;
   ok &= dalloc(c->d_queue, 8) == cudaSuccess;
-  ok &= dalloc(c->d_warp_events, N) == cudaSuccess;
-  ok &= dalloc(c->d_block_events, N) == cudaSuccess;
   ok &= dalloc(c->d_event_order, N) == cudaSuccess;
   ok &= cudaMallocHost(reinterpret_cast<void**>(&c->h_totals), 4 * sizeof(uint32_t) + 8) == cudaSuccess;
   ok &= cudaMallocHost(reinterpret_cast<void**>(&c->h_offsets), 3 * (static_cast<size_t>(N) + 1) * sizeof(uint64_t)) ==
@@ -564,10 +551,6 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   size_search_grid(c);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gec_count_kernel, kGecThreads, 0);
   c->gec_blocks = static_cast<uint32_t>(std::max(1, occ) * c->sm_count);
-  cudaFuncSetAttribute(search_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(kStageCap * sizeof(float4)));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_block_kernel, kBlockThreads, kStageCap * sizeof(float4));
-  c->search_block_blocks = static_cast<uint32_t>(std::max(1, occ) * c->sm_count);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, label_seeds_kernel, kFillThreads, 0);
   c->fill_blocks = static_cast<uint32_t>(std::max(1, occ) * c->sm_count);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, candidate_features_kernel, kFillThreads, 0);
@@ -583,9 +566,9 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   c->score_blocks = static_cast<uint32_t>(score_per_sm * c->sm_count);
   c->mode = cfg->mode == VELO_MODE_PRUNED ? VELO_MODE_PRUNED : VELO_MODE_PLAIN;
   if (c->mode == VELO_MODE_PRUNED && ensure_pruned_buffers(c) != 0) return fail(VELO_ERR_CUDA);
-  // mapping: VELO_MAP_WARP keeps every event on warps, VELO_MAP_BLOCK on blocks; the
-  // default splits at a cluster count (velo_set_block_threshold / the autotuner move it)
-  c->block_threshold = cfg->mapping == VELO_MAP_WARP ? kEventHitCap : (cfg->mapping == VELO_MAP_BLOCK ? 0u : 1536u);
+  // mapping: VELO_MAP_BLOCK gives every event a block; otherwise the order kernel's rule decides
+  // (velo_set_block_threshold / the autotuner add a cluster count)
+  c->block_threshold = cfg->mapping == VELO_MAP_BLOCK ? 0u : kEventHitCap;
   if (cudaGetLastError() != cudaSuccess) return fail(VELO_ERR_CUDA);
   *out = c;
   return 0;

@@ -695,9 +695,6 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
       P.event_hit_base[e] = base;
       P.event_hits[e] = nhits;
       P.status[e] = sh.flags;
-      // route the event to the search mapping chosen for its size
-      if (nhits > P.block_threshold) P.block_events[atomicAdd(P.queue + 5, 1u)] = e;
-      else P.warp_events[atomicAdd(P.queue + 4, 1u)] = e;
     }
     __syncthreads();
   }

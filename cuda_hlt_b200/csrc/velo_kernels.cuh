@@ -137,13 +137,12 @@ struct ChainPointers {
   uint32_t max_tracks_total;
   uint32_t max_track_hits_total;
   uint64_t hit_capacity;       // entries of the hit SoA arrays
-  // work queues: [0] decode, [1] warp search, [2] block search, [3] fill_candidates,
-  // [4] / [5] sizes of the warp / block event lists, [6] error bits, [7] candidate rows
+  // work queues: [0] decode, [1] warp search, [2] block search, [5] events of the block
+  // search, [6] error bits, [7] candidate rows
   uint32_t* queue;             // [8]
-  uint32_t* warp_events;       // [N] events routed to the warp-per-event search
-  uint32_t* event_order;       // [N] warp_events, largest first: the warp search's queue order
-  uint32_t* block_events;      // [N] events routed to the block-per-event search
-  uint32_t block_threshold;    // events with more clusters than this go to the block search
+  uint32_t* event_order;       // [N] events, largest first: the search's queue order
+  uint32_t block_threshold;    // events with more clusters than this take a block in the search
+  uint32_t search_warps;       // resident warps of the search
   // learned pruning (read when keep != nullptr)
   MlpDevice mlp;
 };

@@ -1,5 +1,6 @@
-// Kernel 3 of the chain: search_by_triplet, one warp per event (persistent, queue), events
-// handed out largest first (order_events_kernel, velo_order.cuh).
+// Kernel 3 of the chain: search_by_triplet, one warp per event, or a block of four for the
+// largest of a batch (persistent, queues), events handed out largest first
+// (order_events_kernel, velo_order.cuh).
 //
 // The module loop, forwarding and weak-track rules are those of the reference
 // (ProcessModules.cu:8-163, TrackForwarding.cu:41-181, TrackSeeding.cu:7-200,
@@ -56,11 +57,6 @@ __device__ __forceinline__ bool seed_triplet(const float4 h0, const float4 h1, c
   const float scatterNum = (dx * dx) + (dy * dy);
   scatter = scatterNum * scatterDenom2;
   return fabsf(dx) < kTolerance && fabsf(dy) < kTolerance && scatter < kMaxScatterSeeding;
-}
-
-__device__ __forceinline__ bool seed_scatter(const float4 h0, const float4 h1, const float4 h2, float& scatter)
-{
-  return seed_slope(h0, h1) && seed_triplet(h0, h1, h2, scatter);
 }
 
 // Forwarding fit of one candidate (TrackForwarding.cu:12-35).
@@ -331,19 +327,69 @@ __device__ __forceinline__ void seed_flush(SeedSlots& sl, uint32_t nc, const flo
   __syncwarp();
 }
 
-// Forwarding reads the phi of its two target modules from shared memory, one after the other
-// in a staging area that reuses the seeding slots (the two phases never overlap).
-constexpr uint32_t kFwdStage = sizeof(SeedSlots) / sizeof(float);
-
-struct SearchWarpShared {
+// Shared state of one event searched by G warps. Forwarding reads the phi of its two target
+// modules from shared memory, one after the other in a staging area that reuses the seeding
+// slots (the two phases never overlap).
+template<int G>
+struct SearchShared {
+  static constexpr uint32_t kFwdStage = G * sizeof(SeedSlots) / sizeof(float);
+  union {
+    SeedSlots seed[G];  // one per warp
+    float fphi[kFwdStage];
+  } u;
   uint32_t used[kEventHitCap / 32];
   uint32_t mstart[kModules];
   uint32_t mnum[kModules];
-  union {
-    SeedSlots seed;
-    float fphi[kFwdStage];
-  } u;
+  uint32_t count[2][G];  // counts of the warps (group_rank), two in turn
+  uint32_t sum;          // OR of the flags and sum of the track hits at the end
+  uint32_t flags;
 };
+
+// The G warps that search one event: one warp, or the G warps of a block.
+template<int G>
+__device__ __forceinline__ uint32_t group_thread()
+{
+  return G == 1 ? lane_id() : threadIdx.x;
+}
+template<int G>
+__device__ __forceinline__ void group_sync()
+{
+  if (G == 1) __syncwarp();
+  else __syncthreads();
+}
+
+// Exclusive rank of each thread over the group for three predicates (each count <= 32 G fits 10
+// bits), and the totals. `turn` alternates between two count buffers, so one barrier a call
+// suffices: a buffer is written again only after the barrier of the call between.
+template<int G>
+__device__ __forceinline__ void group_rank(SearchShared<G>& sh, uint32_t& turn, bool p0, bool p1, bool p2,
+                                           uint32_t (&rank)[3], uint32_t (&total)[3])
+{
+  const uint32_t lt = (1u << lane_id()) - 1u;
+  const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, p0), b1 = __ballot_sync(0xFFFFFFFFu, p1),
+                 b2 = __ballot_sync(0xFFFFFFFFu, p2);
+  uint32_t before = 0, all = __popc(b0) | (__popc(b1) << 10) | (__popc(b2) << 20);
+  if constexpr (G > 1) {
+    static_assert(32 * G < 1024, "counts of 10 bits");
+    const uint32_t warp = threadIdx.x >> 5;
+    if (lane_id() == 0) sh.count[turn][warp] = all;
+    __syncthreads();
+    all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < G; ++w) {
+      const uint32_t v = sh.count[turn][w];
+      before += w < warp ? v : 0u;
+      all += v;
+    }
+    turn ^= 1u;
+  }
+  rank[0] = (before & 0x3FFu) + __popc(b0 & lt);
+  rank[1] = ((before >> 10) & 0x3FFu) + __popc(b1 & lt);
+  rank[2] = (before >> 20) + __popc(b2 & lt);
+  total[0] = all & 0x3FFu;
+  total[1] = (all >> 10) & 0x3FFu;
+  total[2] = all >> 20;
+}
 
 // phi window of a forwarded track in one module (TrackForwarding.cuh:28-59), with the
 // module's phi staged in shared memory (`sphi`, null when the module did not fit): the
@@ -425,7 +471,7 @@ __device__ __forceinline__ float forward_best(const float4* H, const uint8_t* KE
   return best_fit;
 }
 
-// Per-event scratch of the warp search: the reference's Velo::TrackHits slots and the rings
+// Per-event scratch of the search: the reference's Velo::TrackHits slots and the rings
 // of tracklets, of tracks to follow and of weak tracklets (SearchByTripletVisitor.cu:11-18).
 struct EventScratch {
   uint16_t* track_n;     // [kMaxTracks]
@@ -460,35 +506,42 @@ struct ComputedWindows {
   }
 };
 
-// Loads the module table of one event into the warp's shared state and clears its used-hit
+// Loads the module table of one event into the group's shared state and clears its used-hit
 // bitmask. module_start holds absolute hit indices; base is the event's first hit.
-__device__ __forceinline__ void search_event_setup(SearchWarpShared& sw, const uint32_t* module_start,
+template<int G>
+__device__ __forceinline__ void search_event_setup(SearchShared<G>& sh, const uint32_t* module_start,
                                                    const uint32_t* module_num, uint32_t base, uint32_t nhits)
 {
-  const uint32_t lane = lane_id();
-  for (uint32_t i = lane; i < (nhits + 31) / 32; i += 32) sw.used[i] = 0u;
-  for (uint32_t m = lane; m < kModules; m += 32) {
-    sw.mstart[m] = module_start[m] - base;
-    sw.mnum[m] = module_num[m];
+  const uint32_t tid = group_thread<G>();
+  for (uint32_t i = tid; i < (nhits + 31) / 32; i += 32 * G) sh.used[i] = 0u;
+  for (uint32_t m = tid; m < kModules; m += 32 * G) {
+    sh.mstart[m] = module_start[m] - base;
+    sh.mnum[m] = module_num[m];
   }
-  __syncwarp();
+  if (tid == 0) {
+    sh.sum = 0;
+    sh.flags = 0;
+  }
+  group_sync<G>();
 }
 
-// search_by_triplet and weak_tracks_adder of one event by one warp (ProcessModules.cu:37-162,
+// search_by_triplet and weak_tracks_adder of one event by G warps (ProcessModules.cu:37-162,
 // TrackSeeding.cu:7-200, TrackForwarding.cu:41-181, WeakTracksAdder.cu:88-115), after
 // search_event_setup. H: the event's phi-sorted cluster records; windows(h1, module): the
 // seeding windows of h1; KE: extension-keep bits per hit (bit 1), or null. Returns the
 // number of tracks written to sc.track_n / sc.track_hits; status bits go to `flags` (per
-// lane: OR-reduce them over the warp).
-template<class Windows>
-__device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, const float4* H, const Windows& windows,
-                                                      const uint8_t* KE, const EventScratch& sc, uint32_t& flags)
+// thread: OR-reduce them over the group). Every append is ranked in the order of one warp
+// taking the work from the front, so the result does not depend on G.
+template<int G, class Windows>
+__device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const float4* H, const Windows& windows,
+                                                 const uint8_t* KE, const EventScratch& sc, uint32_t& flags)
 {
-  const uint32_t lane = lane_id();
-  uint32_t* used = sw.used;
-  uint32_t* mstart = sw.mstart;
-  uint32_t* mnum = sw.mnum;
-  SeedSlots& sl = sw.u.seed;
+  const uint32_t lane = lane_id(), tid = group_thread<G>();
+  const uint32_t warp = G == 1 ? 0u : threadIdx.x >> 5;
+  uint32_t* used = sh.used;
+  const uint32_t* mstart = sh.mstart;
+  const uint32_t* mnum = sh.mnum;
+  SeedSlots& sl = sh.u.seed[warp];
   uint16_t* track_n = sc.track_n;
   uint16_t* track_hits = sc.track_hits;
   uint16_t* tracklets = sc.tracklets;
@@ -496,86 +549,48 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
   uint16_t* weak = sc.weak;
   uint32_t n_tracks = 0, tracklet_ptr = 0, ttf_ptr = 0, weak_ptr = 0;
   uint32_t last_seeded = 0;
+  uint32_t turn = 0;
 
   // ---- seeding: h1 in modules first-2 / first-3, h0 in h1+2, h2 in h1-2 ----
+  // The two modules' seeds are independent (seeding marks no hit used). One warp takes the
+  // modules' h1 in turn (first - 2, then first - 3), queueing unused ones with windows until
+  // kSeedChunk wait: a module's last few hits share a pass with the next module's first ones.
+  // G warps take G equal runs of both modules' h1, at most kSeedChunk each, at a time, and
+  // append their winners run after run.
   auto seeding = [&](uint32_t first) {
     uint32_t n_h1 = 0;
     const uint32_t tracklets_before = tracklet_ptr;
-    // Candidates of both modules (first - 2, then first - 3) are queued in the slots and
-    // processed kSeedChunk at a time: a module's last few hits share a pass with the next
-    // module's first ones. The two modules' seeds are independent (seeding marks no hit
-    // used), and winners are appended in queue order, the order of a pass per module.
-    uint32_t nc = 0;  // candidates queued
-    auto flush = [&]() {
-      seed_flush(sl, nc, H, used);
-      // winners, appended in candidate order (TrackSeeding.cu:185-195)
-      for (uint32_t k0 = 0; k0 < nc; k0 += 32) {
-        const uint32_t k = k0 + lane;
-        const bool win = k < nc && sl.best[k] != ~0ull;
-        uint32_t nwin;
-        const uint32_t rank = ballot_rank(win, nwin);
-        if (win) {
-          const unsigned long long key = sl.best[k];
-          if (static_cast<uint32_t>(key >> 32) == sl.tie[k]) flags |= kStatusSeedTie;
-          const uint32_t tp = (tracklet_ptr + rank) % kTrackletRing;
-          tracklets[3 * tp] = static_cast<uint16_t>(sl.f0[k] + ((key >> 16) & 0xFFFFu));
-          tracklets[3 * tp + 1] = sl.h1[k];
-          tracklets[3 * tp + 2] = static_cast<uint16_t>(sl.f2[k] + (key & 0xFFFFu));
-          ttf[(ttf_ptr + rank) % kTtfModulo] = 0x80000000u | tp;
-        }
-        tracklet_ptr += nwin;
-        ttf_ptr += nwin;
-      }
-      __syncwarp();
-      nc = 0;
-    };
-    int side = 2;
-    uint32_t r0 = 0;
-    for (;;) {
-      while (side <= 3 && r0 >= mnum[first - side]) {
-        ++side;
-        r0 = 0;
-      }
-      const bool have = side <= 3;
-      // (a) unused h1 with both phi windows (FillCandidates.cu:31-68, TrackSeeding.cu:24-49)
-      // among the next (up to) kSeedChunk hits; the windows of their 32-hit groups are
-      // loaded together so that their latencies overlap
-      uint32_t start = 0, r_end = 0, n_new = 0;
-      uint2 wv[kSeedChunk / 32];
-      bool hv[kSeedChunk / 32];
+    uint32_t nc = 0;  // candidates queued by this warp
+    uint2 wv[kSeedChunk / 32];
+    bool hv[kSeedChunk / 32];
+    // the next (up to) kSeedChunk h1, hit_of(r) for r in [r0, r_end): unused, with both phi
+    // windows (FillCandidates.cu:31-68, TrackSeeding.cu:24-49); the windows of their 32-hit
+    // groups are loaded together so that their latencies overlap
+    auto gather = [&](uint32_t r0, uint32_t r_end, auto hit_of, auto module_of) {
+      uint32_t n_new = 0;
 #pragma unroll
       for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
+        const uint32_t r = r0 + 32 * j + lane;
         wv[j] = make_uint2(0xFFFFu, 0xFFFFu);
-        hv[j] = false;
+        if (r < r_end && !test_used(used, hit_of(r))) wv[j] = windows(hit_of(r), module_of(r));
       }
-      if (have) {
-        const uint32_t m = first - side;
-        start = mstart[m];
-        r_end = min(mnum[m], r0 + kSeedChunk);
-#pragma unroll
-        for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
-          const uint32_t r = r0 + 32 * j + lane;
-          if (r < r_end && !test_used(used, start + r)) wv[j] = windows(start + r, m);
-        }
-#pragma unroll
-        for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
-          const uint32_t r = r0 + 32 * j + lane;
-          hv[j] = r < r_end && (wv[j].x & 0xFFFFu) != 0xFFFFu && (wv[j].y & 0xFFFFu) != 0xFFFFu;
-          n_new += __popc(__ballot_sync(0xFFFFFFFFu, hv[j]));
-        }
-      }
-      if (nc > 0 && (!have || nc + n_new > kSeedChunk)) flush();
-      if (!have) break;
 #pragma unroll
       for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
-        const uint32_t h1 = start + r0 + 32 * j + lane;
-        const uint2 w = wv[j];
+        const uint32_t r = r0 + 32 * j + lane;
+        hv[j] = r < r_end && (wv[j].x & 0xFFFFu) != 0xFFFFu && (wv[j].y & 0xFFFFu) != 0xFFFFu;
+        n_new += __popc(__ballot_sync(0xFFFFFFFFu, hv[j]));
+      }
+      return n_new;
+    };
+    auto queue = [&](uint32_t r0, auto hit_of) {
+#pragma unroll
+      for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
         uint32_t cnt;
         const uint32_t rank = ballot_rank(hv[j], cnt);
         if (hv[j]) {
           const uint32_t k = nc + rank;
-          const uint32_t f0 = w.x & 0xFFFFu, l0 = w.x >> 16, f2 = w.y & 0xFFFFu, l2 = w.y >> 16;
-          sl.h1[k] = static_cast<uint16_t>(h1);
+          const uint32_t f0 = wv[j].x & 0xFFFFu, l0 = wv[j].x >> 16, f2 = wv[j].y & 0xFFFFu, l2 = wv[j].y >> 16;
+          sl.h1[k] = static_cast<uint16_t>(hit_of(r0 + 32 * j + lane));
           sl.f0[k] = static_cast<uint16_t>(f0);
           sl.f2[k] = static_cast<uint16_t>(f2);
           sl.n2[k] = static_cast<uint16_t>(l2 - f2);
@@ -585,8 +600,83 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
         }
         nc += cnt;
       }
-      n_h1 += n_new;
-      r0 += kSeedChunk;
+    };
+    // winners of this warp's queue, appended in candidate order from position `at` on
+    // (TrackSeeding.cu:185-195)
+    auto append = [&](uint32_t at) {
+      for (uint32_t k0 = 0; k0 < nc; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        const bool win = k < nc && sl.best[k] != ~0ull;
+        uint32_t nwin;
+        const uint32_t rank = at + ballot_rank(win, nwin);
+        if (win) {
+          const unsigned long long key = sl.best[k];
+          if (static_cast<uint32_t>(key >> 32) == sl.tie[k]) flags |= kStatusSeedTie;
+          const uint32_t tp = (tracklet_ptr + rank) % kTrackletRing;
+          tracklets[3 * tp] = static_cast<uint16_t>(sl.f0[k] + ((key >> 16) & 0xFFFFu));
+          tracklets[3 * tp + 1] = sl.h1[k];
+          tracklets[3 * tp + 2] = static_cast<uint16_t>(sl.f2[k] + (key & 0xFFFFu));
+          ttf[(ttf_ptr + rank) % kTtfModulo] = 0x80000000u | tp;
+        }
+        at += nwin;
+      }
+      __syncwarp();
+      nc = 0;
+      return at;
+    };
+    if constexpr (G == 1) {
+      int side = 2;
+      uint32_t r0 = 0;
+      for (;;) {
+        while (side <= 3 && r0 >= mnum[first - side]) {
+          ++side;
+          r0 = 0;
+        }
+        const bool have = side <= 3;
+        const uint32_t m = first - (have ? side : 3);
+        const uint32_t start = mstart[m];
+        auto hit_of = [&](uint32_t r) { return start + r; };
+        const uint32_t n_new = gather(r0, have ? min(mnum[m], r0 + kSeedChunk) : 0u, hit_of, [&](uint32_t) { return m; });
+        if (nc > 0 && (!have || nc + n_new > kSeedChunk)) {
+          seed_flush(sl, nc, H, used);
+          const uint32_t n = append(0);
+          tracklet_ptr += n;
+          ttf_ptr += n;
+        }
+        if (!have) break;
+        queue(r0, hit_of);
+        n_h1 += n_new;
+        r0 += kSeedChunk;
+      }
+    } else {
+      const uint32_t ma = first - 2, mb = first - 3;
+      const uint32_t na = mnum[ma], n_list = na + mnum[mb], sa = mstart[ma], sb = mstart[mb] - na;
+      auto hit_of = [&](uint32_t r) { return (r < na ? sa : sb) + r; };
+      for (uint32_t r0 = 0; r0 < n_list; r0 += G * kSeedChunk) {
+        const uint32_t run = (min(n_list - r0, G * kSeedChunk) + G - 1) / G;
+        const uint32_t lo = min(n_list, r0 + warp * run), hi = min(n_list, lo + run);
+        const uint32_t n_new = gather(lo, hi, hit_of, [&](uint32_t r) { return r < na ? ma : mb; });
+        queue(lo, hit_of);
+        if (nc > 0) seed_flush(sl, nc, H, used);
+        uint32_t nwin = 0;
+        for (uint32_t k0 = 0; k0 < nc; k0 += 32)
+          nwin += __popc(__ballot_sync(0xFFFFFFFFu, k0 + lane < nc && sl.best[k0 + lane] != ~0ull));
+        if (lane == 0) sh.count[turn][warp] = nwin | (n_new << 16);
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < G; ++w) {
+          const uint32_t v = sh.count[turn][w];
+          before += w < warp ? v : 0u;
+          all += v;
+        }
+        turn ^= 1u;
+        append(before & 0xFFFFu);
+        tracklet_ptr += all & 0xFFFFu;
+        ttf_ptr += all & 0xFFFFu;
+        n_h1 += all >> 16;
+      }
+      __syncthreads();  // the appended seeds, and the slots before they are staged over
     }
     if (n_h1 > kMaxHitsPerModule) flags |= kStatusH1Overflow;
     const uint32_t seeded = tracklet_ptr - tracklets_before;
@@ -601,16 +691,16 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
     const float moz = c_module_z[mo], mez = c_module_z[me];
     // stage the phi of both target modules (their searches then stay in shared memory); a pair
     // of modules above the staging size is searched in global memory
-    const bool fits = mon + men <= kFwdStage;
-    const float* sphi_o = fits ? sw.u.fphi : nullptr;
-    const float* sphi_e = fits ? sw.u.fphi + mon : nullptr;
+    const bool fits = mon + men <= SearchShared<G>::kFwdStage;
+    const float* sphi_o = fits ? sh.u.fphi : nullptr;
+    const float* sphi_e = fits ? sh.u.fphi + mon : nullptr;
     if (diff > 0 && fits) {
-      for (uint32_t i = lane; i < mon; i += 32) sw.u.fphi[i] = H[mos + i].w;
-      for (uint32_t i = lane; i < men; i += 32) sw.u.fphi[mon + i] = H[mes + i].w;
+      for (uint32_t i = tid; i < mon; i += 32 * G) sh.u.fphi[i] = H[mos + i].w;
+      for (uint32_t i = tid; i < men; i += 32 * G) sh.u.fphi[mon + i] = H[mes + i].w;
     }
-    __syncwarp();
-    for (uint32_t i0 = 0; i0 < diff; i0 += 32) {
-      const uint32_t i = i0 + lane;
+    group_sync<G>();
+    for (uint32_t i0 = 0; i0 < diff; i0 += 32 * G) {
+      const uint32_t i = i0 + tid;
       int action = 0;  // 1 extend, 2 keep with a skipped module, 3 demote to weak
       uint32_t full = 0, trackno = 0, nhit = 0;
       uint16_t t0 = 0, t1 = 0, t2 = 0, best_h2 = 0;
@@ -657,11 +747,16 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
           set_used(used, t2);
         }
       }
-      uint32_t n_new;
-      const uint32_t new_rank = ballot_rank(action == 1 && nhit == 3, n_new);
+      const bool is_new = action == 1 && nhit == 3;
+      uint32_t rank[3], total[3];  // new tracks, tracks followed on, weak tracklets
+      group_rank<G>(sh, turn, is_new, action == 1 || action == 2, action == 3, rank, total);
+      // new tracks beyond the last slot are dropped, and not followed
+      const uint32_t slot = n_tracks + rank[0];
+      const uint32_t dropped = slot > kMaxTracks ? slot - kMaxTracks : 0u;  // before this thread's
+      const uint32_t all_tracks = n_tracks + total[0];
+      const uint32_t all_dropped = all_tracks > kMaxTracks ? all_tracks - kMaxTracks : 0u;
       bool stored = action == 1;
-      if (action == 1 && nhit == 3) {
-        const uint32_t slot = n_tracks + new_rank;
+      if (is_new) {
         if (slot < kMaxTracks) {
           uint16_t* th = track_hits + slot * kMaxTrackSize;
           th[0] = t0;
@@ -677,28 +772,23 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
         track_hits[trackno * kMaxTrackSize + nhit] = best_h2;
         track_n[trackno] = static_cast<uint16_t>(nhit + 1);
       }
-      if (n_tracks + n_new > kMaxTracks) flags |= kStatusTrackOverflow;
-      n_tracks = min(n_tracks + n_new, kMaxTracks);
-      const bool push = stored || action == 2;
-      uint32_t n_push;
-      const uint32_t push_rank = ballot_rank(push, n_push);
-      if (push) {
+      if (all_dropped) flags |= kStatusTrackOverflow;
+      n_tracks = all_tracks - all_dropped;
+      if (stored || action == 2) {
         const uint32_t value =
           action == 2 ? ((((full & 0x70000000u) >> 28) + 1) << 28) | (full & 0x8FFFFFFFu) : trackno;
-        ttf[(ttf_ptr + push_rank) % kTtfModulo] = value;
+        ttf[(ttf_ptr + rank[1] - dropped) % kTtfModulo] = value;
       }
-      ttf_ptr += n_push;
-      uint32_t n_weak;
-      const uint32_t weak_rank = ballot_rank(action == 3, n_weak);
-      if (action == 3 && weak_ptr + weak_rank < kWeakCap) {
-        uint16_t* w = weak + 3 * (weak_ptr + weak_rank);
+      ttf_ptr += total[1] - all_dropped;
+      if (action == 3 && weak_ptr + rank[2] < kWeakCap) {
+        uint16_t* w = weak + 3 * (weak_ptr + rank[2]);
         w[0] = t0;
         w[1] = t1;
         w[2] = t2;
       }
-      weak_ptr += n_weak;
+      weak_ptr += total[2];
     }
-    __syncwarp();
+    group_sync<G>();
   };
 
   // ---- module loop (ProcessModules.cu:37-162) ----
@@ -719,29 +809,29 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
     // tracklets still waiting become weak (ProcessModules.cu:146-162)
     const uint32_t prev = last_ttf;
     const uint32_t diff = ttf_ptr - prev;
-    for (uint32_t i0 = 0; i0 < diff; i0 += 32) {
-      const uint32_t i = i0 + lane;
+    for (uint32_t i0 = 0; i0 < diff; i0 += 32 * G) {
+      const uint32_t i = i0 + tid;
       uint32_t full = 0;
       if (i < diff) full = ttf[(prev + i) % kTtfModulo];
       const bool is_weak = i < diff && (full & 0x80000000u);
-      uint32_t n_weak;
-      const uint32_t rank = ballot_rank(is_weak, n_weak);
-      if (is_weak && weak_ptr + rank < kWeakCap) {
+      uint32_t rank[3], total[3];
+      group_rank<G>(sh, turn, is_weak, false, false, rank, total);
+      if (is_weak && weak_ptr + rank[0] < kWeakCap) {
         const uint32_t tp = full & 0x0FFFFFFFu;
-        uint16_t* w = weak + 3 * (weak_ptr + rank);
+        uint16_t* w = weak + 3 * (weak_ptr + rank[0]);
         w[0] = tracklets[3 * tp];
         w[1] = tracklets[3 * tp + 1];
         w[2] = tracklets[3 * tp + 2];
       }
-      weak_ptr += n_weak;
+      weak_ptr += total[0];
     }
   }
   if (weak_ptr > kMaxWeakTracks) flags |= kStatusWeakOverflow;
-  __syncwarp();
+  group_sync<G>();
   // ---- weak_tracks_adder (WeakTracksAdder.cu:88-115) ----
   const uint32_t n_weak = min(weak_ptr, kWeakCap);
-  for (uint32_t i0 = 0; i0 < n_weak; i0 += 32) {
-    const uint32_t i = i0 + lane;
+  for (uint32_t i0 = 0; i0 < n_weak; i0 += 32 * G) {
+    const uint32_t i = i0 + tid;
     bool accept = false;
     uint16_t h[3] = {0, 0, 0};
     if (i < n_weak) {
@@ -752,10 +842,10 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
       const float chi2 = weak_chi2(H, h);
       accept = !any_used && chi2 < kMaxChi2;
     }
-    uint32_t n_acc;
-    const uint32_t rank = ballot_rank(accept, n_acc);
+    uint32_t rank[3], total[3];
+    group_rank<G>(sh, turn, accept, false, false, rank, total);
     if (accept) {
-      const uint32_t slot = n_tracks + rank;
+      const uint32_t slot = n_tracks + rank[0];
       if (slot < kMaxTracks) {
         uint16_t* th = track_hits + slot * kMaxTrackSize;
         th[0] = h[0];
@@ -764,59 +854,94 @@ __device__ __forceinline__ uint32_t search_event_warp(SearchWarpShared& sw, cons
         track_n[slot] = 3;
       }
     }
-    if (n_tracks + n_acc > kMaxTracks) flags |= kStatusTrackOverflow;
-    n_tracks = min(n_tracks + n_acc, kMaxTracks);
+    if (n_tracks + total[0] > kMaxTracks) flags |= kStatusTrackOverflow;
+    n_tracks = min(n_tracks + total[0], kMaxTracks);
   }
-  __syncwarp();
+  group_sync<G>();
   return n_tracks;
 }
 
+// One event of the chain by G warps: its tracks, their count and hit count and its status.
+template<int G>
+__device__ __forceinline__ void search_chain_event(SearchShared<G>& sh, const ChainPointers& P, uint32_t e)
+{
+  const uint32_t lane = lane_id(), tid = group_thread<G>();
+  const uint32_t nhits = P.event_hits[e];
+  const uint32_t status = P.status[e];
+  const uint32_t base = P.event_hit_base[e];
+  uint32_t flags = 0;  // per thread, OR-reduced at the end
+  uint32_t n_tracks = 0, track_hits = 0;
+  const bool runnable = !(status & (kStatusBadRawEvent | kStatusHitOverflow)) && nhits <= kEventHitCap && nhits > 0;
+  if (nhits > kEventHitCap) flags |= kStatusHitOverflow;
+  if (runnable) {
+    search_event_setup<G>(sh, P.module_start + e * kModules, P.module_num + e * kModules, base, nhits);
+    const EventScratch sc{P.scratch.track_n + static_cast<size_t>(e) * kMaxTracks,
+                          P.scratch.track_hits + static_cast<size_t>(e) * kMaxTracks * kMaxTrackSize,
+                          P.scratch.tracklets + static_cast<size_t>(e) * kTrackletRing * 3,
+                          P.scratch.ttf + static_cast<size_t>(e) * kTtfModulo,
+                          P.scratch.weak + static_cast<size_t>(e) * kWeakCap * 3};
+    const uint8_t* KE = (P.keep && P.mlp.use_ext) ? P.keep + base : nullptr;  // extension pruning
+    n_tracks = search_event<G>(sh, P.hits.xyzp + base, StoredWindows{P.windows + base}, KE, sc, flags);
+    for (uint32_t t = tid; t < n_tracks; t += 32 * G) track_hits += sc.track_n[t];
+  }
+  flags = __reduce_or_sync(0xFFFFFFFFu, flags);
+  track_hits = __reduce_add_sync(0xFFFFFFFFu, track_hits);
+  if (G > 1 && runnable) {
+    if (lane == 0) {
+      atomicOr(&sh.flags, flags);
+      atomicAdd(&sh.sum, track_hits);
+    }
+    __syncthreads();
+    flags = sh.flags;
+    track_hits = sh.sum;
+  }
+  if (tid == 0) {
+    P.event_tracks[e] = n_tracks;
+    P.event_track_hits[e] = track_hits;
+    P.status[e] = status | flags;
+  }
+  group_sync<G>();
+}
+
+// Persistent; the events largest first (order_events_kernel). The first queue[5] of them take
+// a whole block, four warps an event, the others a warp each: a warp's events follow one
+// another, so an event that alone takes longer than a warp's share of the batch would set the
+// kernel's length. Four warps search an event in less than half of a warp's time (the module
+// steps' barriers and part-filled rounds take the rest), so a batch that fills the device with
+// events keeps to one warp each. Against one warp per event throughout: search of 1,000 events
+// at nu = 7.6 0.64 -> 0.28 ms, of 3,000 at nu = 15 with noise 5.95 -> 1.79 ms, of 8,191 at
+// nu ~ U(2,20) with every candidate scored 2.50 -> 1.32 ms; of 65,536, where no event takes a
+// block, 13.35 -> 13.17 ms.
+//
 // 8 blocks of 4 warps per SM at 64 registers: more resident events (10 or 12 blocks at 48 or
 // 40 registers) measured slower, their hit records competing for L1.
-template<int WPB>
-__global__ void __launch_bounds__(WPB * 32, 8) search_kernel(ChainPointers P)
+constexpr int kSearchWarps = 4;
+
+template<int W>
+__global__ void __launch_bounds__(W * 32, 32 / W) search_kernel(ChainPointers P)
 {
-  __shared__ SearchWarpShared s_warp[WPB];
-  const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
-  SearchWarpShared& sw = s_warp[warp];
+  __shared__ union {
+    SearchShared<W> block;
+    SearchShared<1> warp[W];
+  } s;
+  __shared__ uint32_t s_next;
+  const uint32_t lane = lane_id();
+  const uint32_t n_events = P.run->n_events, n_block = P.queue[5];
 
   for (;;) {
+    if (threadIdx.x == 0) s_next = atomicAdd(P.queue + 2, 1u);
+    __syncthreads();
+    const uint32_t q = s_next;
+    __syncthreads();
+    if (q >= n_block) break;
+    search_chain_event<W>(s.block, P, P.event_order[q]);
+  }
+  for (;;) {
     uint32_t q = 0;
-    if (lane == 0) q = atomicAdd(P.queue + 1, 1u);
+    if (lane == 0) q = n_block + atomicAdd(P.queue + 1, 1u);
     q = __shfl_sync(0xFFFFFFFFu, q, 0);
-    if (q >= P.queue[4]) break;
-    const uint32_t e = P.event_order[q];
-    const uint32_t nhits = P.event_hits[e];
-    const uint32_t status = P.status[e];
-    const uint32_t base = P.event_hit_base[e];
-    uint32_t flags = 0;  // per lane, OR-reduced at the end
-    uint32_t n_tracks = 0, total_hits_on_tracks = 0;
-    const bool runnable = !(status & (kStatusBadRawEvent | kStatusHitOverflow)) && nhits <= kEventHitCap && nhits > 0;
-    if (nhits > kEventHitCap) flags |= kStatusHitOverflow;
-    if (runnable) {
-      search_event_setup(sw, P.module_start + e * kModules, P.module_num + e * kModules, base, nhits);
-      const EventScratch sc{P.scratch.track_n + static_cast<size_t>(e) * kMaxTracks,
-                            P.scratch.track_hits + static_cast<size_t>(e) * kMaxTracks * kMaxTrackSize,
-                            P.scratch.tracklets + static_cast<size_t>(e) * kTrackletRing * 3,
-                            P.scratch.ttf + static_cast<size_t>(e) * kTtfModulo,
-                            P.scratch.weak + static_cast<size_t>(e) * kWeakCap * 3};
-      const uint8_t* KE = (P.keep && P.mlp.use_ext) ? P.keep + base : nullptr;  // extension pruning
-      n_tracks = search_event_warp(sw, P.hits.xyzp + base, StoredWindows{P.windows + base}, KE, sc, flags);
-      uint32_t sum = 0;
-      for (uint32_t t = lane; t < n_tracks; t += 32) sum += sc.track_n[t];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-      total_hits_on_tracks = sum;
-    }
-    uint32_t f = flags;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) f |= __shfl_xor_sync(0xFFFFFFFFu, f, o);
-    if (lane == 0) {
-      P.event_tracks[e] = runnable ? n_tracks : 0;
-      P.event_track_hits[e] = runnable ? total_hits_on_tracks : 0;
-      P.status[e] = status | f;
-    }
-    __syncwarp();
+    if (q >= n_events) break;
+    search_chain_event<1>(s.warp[threadIdx.x >> 5], P, P.event_order[q]);
   }
 }
 

@@ -5,9 +5,8 @@ graphs, default output capacities: 400 tracks per event).
 python -m cuda_hlt_b200.profile_case [--events 8192] [--runs 2] [--block-threshold N] [--mode plain|pruned] [--pv]
                                      [--gec] [--every-candidate]
 
---block-threshold: events with more clusters than N use the block-per-event search, the
-others the warp-per-event one (1536 is the context default; 16384 sends every event to
-the warp search).
+--block-threshold: events with more clusters than N take a block in the search whatever the
+batch (16384, the context default, leaves it to the mapping's own rule).
 --every-candidate: in the pruned mode, the committed scorer with its gates open (every event
 and every seeding candidate scored).
 """
@@ -21,7 +20,7 @@ def main():
     ap.add_argument("--events", type=int, default=8192)
     ap.add_argument("--runs", type=int, default=2)
     ap.add_argument("--config", default="batched_500k")
-    ap.add_argument("--block-threshold", type=int, default=1536)
+    ap.add_argument("--block-threshold", type=int, default=16384)
     ap.add_argument("--mode", default="plain", choices=["plain", "pruned"])
     ap.add_argument("--pv", action="store_true", help="append the beamline PV stage")
     ap.add_argument("--every-candidate", action="store_true",

@@ -158,10 +158,13 @@ typedef struct VeloCtx VeloCtx;
                               (velo_capture_labels): a perfect scorer at no cost, which measures
                               how much pruning can save at most */
 
-/* Search mapping (velo_set_block_threshold sets the boundary directly). */
-#define VELO_MAP_AUTO 0    /* search: block per event above 1,536 clusters, warp per event below */
+/* Search mapping. A warp searches an event, or a block of four warps does: the events above the
+ * boundary of velo_set_block_threshold, and those whose search on one warp would outlast a
+ * warp's share of the batch (a batch too small to fill the device gives every event a
+ * block). The tracks do not depend on it. */
+#define VELO_MAP_AUTO 0    /* search: no boundary */
 #define VELO_MAP_BLOCK 1   /* search: one block per event */
-#define VELO_MAP_WARP 2    /* search: one warp per event */
+#define VELO_MAP_WARP 2    /* search: no boundary */
 
 typedef struct VeloConfig {
   uint32_t max_events;          /* events per velo_run call */
@@ -395,9 +398,9 @@ int velo_download_async(VeloCtx* ctx, void* dst_host, const void* src_device, si
  * default. */
 int velo_set_pv(VeloCtx* ctx, int enabled);
 
-/* Search mapping: events with more than `clusters` clusters run the block-per-event search,
- * the others the warp-per-event search (0: all block, >= 16384: all warp). Set by the
- * autotuner (cuda_hlt_b200/autotune.py) from timings per hit-count bucket. */
+/* Search mapping: events with more than `clusters` clusters always take a block in the search
+ * (0: all, >= 16384: none but those the mapping's own rule gives one). Set by the autotuner
+ * (cuda_hlt_b200/autotune.py) from timings per hit-count bucket. */
 int velo_set_block_threshold(VeloCtx* ctx, uint32_t clusters);
 
 /* Decode block size: 4 or 8 warps per event (default 8); set by the autotuner
