@@ -9,9 +9,9 @@
 //     the block then flood-fills with every thread busy;
 //   * clusters go to their module's slice of a staging area sized by the module's SP count
 //     (at most two clusters per SP), one shared atomic per cluster;
-//   * one warp per module sorts the slice on the key (phi, LHCb id) - in registers with
-//     warp shuffles up to 128 clusters, in shared memory up to 512 - and writes it to the
-//     compact phi-sorted layout.
+//   * one warp per module sorts the slice on (phi, LHCb id) - up to 256 clusters in registers
+//     on 32-bit keys with warp shuffles, up to 512 (and where short keys agree) in shared memory
+//     on the full keys - and writes it to the compact phi-sorted layout.
 // The result equals the reference's estimate -> prefix sum -> masked clustering ->
 // calculate_phi_and_sort sequence, whose order within a module depends on the order of its
 // atomics only for exactly equal phi.
@@ -164,7 +164,7 @@ __device__ __forceinline__ bool flood_window(uint32_t px0, uint32_t px1, uint32_
 constexpr uint32_t kCandCap = 4096;    // candidate pixels listed per event (more: flooded inline)
 constexpr uint32_t kBankMapCap = 16384; // SPs per event with a bank map (more: binary search)
 constexpr uint32_t kNonIsoCap = 2048;   // non-isolated SPs listed per event (more: full rescan)
-constexpr uint32_t kRegSortMax = 128;  // modules up to this size are sorted in registers
+constexpr uint32_t kRegSortMax = 256;  // modules up to this size are sorted in registers
 
 struct DecodeShared {
   uint32_t bank_start[kSensors];  // word index (from the event start) of the first SP word
@@ -257,27 +257,37 @@ __device__ __forceinline__ unsigned long long cluster_key(const float4* src, con
          (static_cast<unsigned long long>(src_id[i] & 0xFFFFFu) << 12) | i;
 }
 
-// Compare-exchange of elements a (lower index) and b in bitonic order `up`: one 64-bit
-// comparison and a conditional swap (keys are distinct: the slot is part of the key).
-__device__ __forceinline__ void bitonic_cx(unsigned long long& a, unsigned long long& b, bool up)
+// Short sort key: phi to 24..26 bits above the staging slot (5 + log2 PER bits). phi + 4 is
+// between 0.85 and 10.3, so the float's bit pattern less that of 0.5 orders it in 26 bits;
+// anything else (a NaN) is cut to a value below the padding key.
+template<uint32_t PER>
+__device__ __forceinline__ uint32_t short_key(float phi, uint32_t slot)
 {
-  const bool swap = (b < a) == up;
-  const unsigned long long t = a;
-  a = swap ? b : a;
-  b = swap ? t : b;
+  constexpr uint32_t kSlotBits = PER == 8 ? 8 : PER == 4 ? 7 : PER == 2 ? 6 : 5;
+  constexpr uint32_t kDrop = kSlotBits > 6 ? kSlotBits - 6 : 0;
+  const uint32_t q = min(__float_as_uint(phi + 4.0f) - 0x3F000000u, 0x3FFFFF0u);
+  return ((q >> kDrop) << kSlotBits) | slot;
 }
 
-// Bitonic sort of 32 * PER keys held PER per lane, element lane * PER + j in key[j]
+// Bitonic sort of 32 * PER 32-bit keys held PER per lane, element lane * PER + j in key[j]
 // (the input may sit in any slots: only the sorted order is read back this way). The
 // exchanges between elements less than PER apart stay inside a lane, the others take one
-// shuffle per key; loops unrolled, so every register index is a compile-time constant and
-// the keys stay in registers.
+// shuffle per key; loops unrolled, so every register index is a compile-time constant. Blocks
+// that sort downwards hold their keys complemented, so every exchange is a plain min and max.
 template<uint32_t PER>
-__device__ __forceinline__ void warp_register_sort(unsigned long long (&key)[4])
+__device__ __forceinline__ void warp_register_sort(uint32_t (&key)[PER])
 {
   const uint32_t lane = lane_id();
+  uint32_t held = 0;  // complement of this lane's keys
 #pragma unroll
   for (uint32_t k = 2; k <= 32 * PER; k <<= 1) {
+    if (k >= PER) {
+      const uint32_t want = (lane * PER) & k ? 0xFFFFFFFFu : 0u;  // none in the last merge
+      const uint32_t flip = (k < 32 * PER ? want : 0u) ^ held;
+      held ^= flip;
+#pragma unroll
+      for (uint32_t j = 0; j < PER; ++j) key[j] ^= flip;
+    }
 #pragma unroll
     for (uint32_t d = k >> 1; d > 0; d >>= 1) {
       if (d >= PER) {
@@ -285,21 +295,65 @@ __device__ __forceinline__ void warp_register_sort(unsigned long long (&key)[4])
         const bool lower = (lane & ld) == 0;
 #pragma unroll
         for (uint32_t j = 0; j < PER; ++j) {
-          const unsigned long long p = __shfl_xor_sync(0xFFFFFFFFu, key[j], ld);
-          const bool up = ((lane * PER + j) & k) == 0;
-          // keep the smaller of the pair (lower lane of an ascending pair, or upper lane of a
-          // descending one) or the larger
-          key[j] = ((p < key[j]) == (lower == up)) ? p : key[j];
+          const uint32_t p = __shfl_xor_sync(0xFFFFFFFFu, key[j], ld);
+          key[j] = (p < key[j]) == lower ? p : key[j];
         }
-      } else if (d == 2) {  // PER == 4: registers j and j + 2
-        bitonic_cx(key[0], key[2], ((lane * PER + 0) & k) == 0);
-        bitonic_cx(key[1], key[3], ((lane * PER + 1) & k) == 0);
-      } else {  // d == 1: registers j and j + 1
-        bitonic_cx(key[0], key[1], ((lane * PER + 0) & k) == 0);
-        if (PER == 4) bitonic_cx(key[2], key[3], ((lane * PER + 2) & k) == 0);
+      } else {
+#pragma unroll
+        for (uint32_t j = 0; j < PER; ++j) {
+          if (j & d) continue;
+          const bool down = k < PER && (j & k);  // a block inside the lane
+          const uint32_t lo = min(key[j], key[j + d]), hi = max(key[j], key[j + d]);
+          key[j] = down ? hi : lo;
+          key[j + d] = down ? lo : hi;
+        }
       }
     }
   }
+}
+
+// Sorts a module's n (<= 32 * PER) staged clusters on (phi, LHCb id) into the compact layout
+// by their short keys. Short keys that agree leave their clusters in slot order: the full keys
+// of neighbours are compared on the way out, and false is returned when one pair stands the
+// wrong way round (about one module in 400): the caller sorts that module on the full keys.
+//
+// Bound by the integer pipe: 32-bit keys take 3 instructions a key and exchange (shuffle,
+// compare, select) where the full 64-bit keys took 9, and 256 of them fit the registers that
+// held 128. Decode of 65,536 events at nu ~ U(2,20) 13.51 -> 11.24 ms.
+template<uint32_t PER>
+__device__ __forceinline__ bool sort_module_short(const float4* src, const uint32_t* src_id, uint32_t n, float4* dst,
+                                                  uint32_t* dst_id, uint8_t* dst_size)
+{
+  const uint32_t lane = lane_id();
+  uint32_t key[PER];
+#pragma unroll
+  for (uint32_t j = 0; j < PER; ++j) {  // coalesced loads
+    const uint32_t i = j * 32 + lane;
+    key[j] = i < n ? short_key<PER>(src[i].w, i) : 0xFFFFFFFFu;
+  }
+  warp_register_sort<PER>(key);
+  bool wrong = false;
+  unsigned long long first = 0, prev = 0;  // full keys without the slot
+#pragma unroll
+  for (uint32_t j = 0; j < PER; ++j) {
+    const uint32_t i = lane * PER + j;  // rank of key[j]
+    unsigned long long full = ~0ull;
+    if (i < n) {
+      const uint32_t from = key[j] & (32 * PER - 1);
+      const uint32_t id = src_id[from];
+      const float4 c = src[from];
+      dst[i] = c;
+      dst_id[i] = id & ~kSizeMask;
+      dst_size[i] = static_cast<uint8_t>(id >> kSizeShift) & 3u;
+      full = (static_cast<unsigned long long>(orderable(c.w)) << 32) | (id & 0xFFFFFu);
+    }
+    if (j == 0) first = full;
+    else wrong |= full < prev;
+    prev = full;
+  }
+  const unsigned long long next = __shfl_down_sync(0xFFFFFFFFu, first, 1);
+  wrong |= lane < 31 && next < prev;
+  return !__any_sync(0xFFFFFFFFu, wrong);
 }
 
 // Bitonic sort of `size` keys (power of two) in shared memory by one warp.
@@ -598,32 +652,18 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
       uint32_t* dst_id = P.hits.id + p0;
       uint8_t* dst_size = P.hit_size + p0;
       if (n > kMaxHitsPerModule && lane == 0) atomicOr(&sh.flags, kStatusModuleOverflow);
-      if (n <= kRegSortMax) {
-        const uint32_t per = n > 64 ? 4 : n > 32 ? 2 : 1;
-        unsigned long long key[4];
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {  // coalesced loads; slots j >= per hold padding only
-          const uint32_t i = j * 32 + lane;
-          key[j] = i < n ? cluster_key(src, src_id, i) : ~0ull;
-        }
-        if (per == 4) warp_register_sort<4>(key);
-        else if (per == 2) warp_register_sort<2>(key);
-        else if (n > 1) warp_register_sort<1>(key);
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-          const uint32_t i = lane * per + j;  // rank of key[j]
-          if (j < per && i < n) {
-            const uint32_t from = static_cast<uint32_t>(key[j] & 0xFFFu);
-            const uint32_t id = src_id[from];
-            dst[i] = src[from];
-            dst_id[i] = id & ~kSizeMask;
-            dst_size[i] = static_cast<uint8_t>(id >> kSizeShift) & 3u;
-          }
-        }
+      bool sorted = n == 0;
+      if (n > 128 && n <= kRegSortMax) sorted = sort_module_short<8>(src, src_id, n, dst, dst_id, dst_size);
+      else if (n > 64 && n <= 128) sorted = sort_module_short<4>(src, src_id, n, dst, dst_id, dst_size);
+      else if (n > 32 && n <= 64) sorted = sort_module_short<2>(src, src_id, n, dst, dst_id, dst_size);
+      else if (n > 0 && n <= 32) sorted = sort_module_short<1>(src, src_id, n, dst, dst_id, dst_size);
+      if (sorted) {
+        // in registers
       } else if (n <= kSortCap) {
         unsigned long long* key = su.key[warp];
-        uint32_t size = 256;
+        uint32_t size = 32;
         while (size < n) size <<= 1;
+        __syncwarp();  // the short keys' order, if any, has been written
         for (uint32_t i = lane; i < size; i += 32) key[i] = i < n ? cluster_key(src, src_id, i) : ~0ull;
         __syncwarp();
         warp_smem_sort(key, size);
