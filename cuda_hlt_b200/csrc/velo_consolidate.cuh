@@ -242,28 +242,37 @@ __device__ __forceinline__ void store_state(char* base, uint32_t T, uint32_t i, 
   reinterpret_cast<bool*>(base + sizeof(float) * 12 * T)[i] = s.backward;
 }
 
-// Consolidation, beamline state and Kalman state of one event per warp. Tracks are
-// taken 32 at a time, one per lane: an exclusive warp scan of their hit counts gives
-// their slices of the output; the hits of the 32 tracks form one contiguous range of the
-// Velo::Consolidated::Hits SoA, which the warp then writes in order (coalesced), each lane
-// finding the track of an output position by binary search over the 32 offsets. The same
-// loop keeps x, y, z of the range in shared memory (up to kConsolidateStage hits), from
-// where the fits run per lane on their track's slice; a larger range (32 tracks averaging
-// more than 16 hits) fits from per-lane copies instead.
+// Consolidation, beamline state and Kalman state, one event per block of W warps, largest
+// events first. The block scans the hit counts of the event's tracks; its warps then take 32
+// tracks at a time, one per lane. The hits of 32 tracks form one contiguous range of the
+// Velo::Consolidated::Hits SoA, which the warp writes in order (coalesced), finding the track
+// of an output position from the starts. The same loop keeps x, y, z of the range in shared
+// memory (up to kConsolidateStage hits), from where the fits run per lane on their track's
+// slice; a larger range (32 tracks averaging more than 16 hits) fits from per-lane copies
+// instead.
+//
+// Bound by the latency of its chain of gathers (hit index, then record and id): a warp per
+// event ran the chain once per 32 tracks, five times over for an average event, and a block
+// waited for the largest of its four events. Four warps an event, of 65,536 at nu ~ U(2,20):
+// 3.75 -> 1.96 ms (two warps: 3.52).
 constexpr uint32_t kConsolidateStage = 512;
+constexpr int kConsolidateWarps = 4;
 
-template<int WPB>
-__global__ void __launch_bounds__(WPB * 32) consolidate_fit_kernel(ChainPointers P)
+template<int W>
+__global__ void __launch_bounds__(W * 32) consolidate_fit_kernel(ChainPointers P)
 {
-  __shared__ uint32_t s_off[WPB][33];
-  __shared__ float s_hit[WPB][3][kConsolidateStage];
+  static_assert(kMaxTracks * kMaxTrackSize < 65536, "hit offsets of an event in 16 bits");
+  __shared__ uint16_t s_off[kMaxTracks + 1];  // first hit of each track in the event
+  __shared__ uint32_t s_warp[W];
+  __shared__ float s_hit[W][3][kConsolidateStage];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const uint32_t e = blockIdx.x * WPB + warp;
   const uint32_t N = P.run->n_events;
-  if (e >= N) return;
+  if (blockIdx.x >= N) return;
+  const uint32_t e = P.event_order[blockIdx.x];
   const uint32_t T = P.atomics[2 * N];
   const uint32_t Htot = P.event_hit_offset[N];
   const uint32_t nt = P.atomics[e];
+  if (nt == 0) return;
   const uint32_t t0 = P.atomics[N + e];
   const float4* H = P.hits.xyzp + P.event_hit_base[e];
   const uint32_t* ids = P.hits.id + P.event_hit_base[e];
@@ -273,28 +282,46 @@ __global__ void __launch_bounds__(WPB * 32) consolidate_fit_kernel(ChainPointers
   uint32_t* oid = reinterpret_cast<uint32_t*>(ox + 3 * static_cast<size_t>(Htot));
   const uint16_t* track_n = P.scratch.track_n + static_cast<size_t>(e) * kMaxTracks;
   const uint16_t* track_hits = P.scratch.track_hits + static_cast<size_t>(e) * kMaxTracks * kMaxTrackSize;
-  uint32_t carry = P.event_hit_offset[e];
-  for (uint32_t i0 = 0; i0 < nt; i0 += 32) {
-    const uint32_t i = i0 + lane;
+  const uint32_t first_hit = P.event_hit_offset[e];
+  // ---- exclusive scan of the hit counts ----
+  uint32_t before = 0;
+  for (uint32_t i0 = 0; i0 < nt; i0 += 32 * W) {
+    const uint32_t i = i0 + threadIdx.x;
     const uint32_t n = i < nt ? track_n[i] : 0;
-    const uint32_t n_chunk = min(32u, nt - i0);  // tracks of this chunk
     uint32_t incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
       if (lane >= static_cast<uint32_t>(o)) incl += v;
     }
-    const uint32_t chunk_hits = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    s_off[warp][lane] = incl - n;
-    if (lane == 31) s_off[warp][32] = incl;
-    __syncwarp();
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t lower = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < W; ++w) {
+      const uint32_t v = s_warp[w];
+      lower += w < warp ? v : 0u;
+      all += v;
+    }
+    if (i < nt) s_off[i] = static_cast<uint16_t>(before + lower + incl - n);
+    before += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) s_off[nt] = static_cast<uint16_t>(before);
+  __syncthreads();
+  // ---- 32 tracks at a time ----
+  for (uint32_t i0 = 32 * warp; i0 < nt; i0 += 32 * W) {
+    const uint32_t i = i0 + lane;
+    const uint32_t n_chunk = min(32u, nt - i0);  // tracks of this chunk
+    const uint32_t chunk0 = s_off[i0], chunk_hits = s_off[i0 + n_chunk] - chunk0;
+    const uint32_t carry = first_hit + chunk0;
     // coalesced write of the chunk's hit range [carry, carry + chunk_hits)
     const bool staged = chunk_hits <= kConsolidateStage;
     // four output positions per lane at a time: their dependent gathers (hit index, then
     // record and id) are in flight together. The track of a position: every track has hits,
     // so the tracks starting inside 32 consecutive positions are marked by one bit each (an
     // OR across the warp of the lanes' own starts) and counted with a popcount.
-    const uint32_t my_start = lane < n_chunk ? s_off[warp][lane] : 0xFFFFFFFFu;
+    const uint32_t my_start = lane < n_chunk ? s_off[i] - chunk0 : 0xFFFFFFFFu;
     uint32_t started = 0;  // tracks starting before the current group of 32 positions
     for (uint32_t base = 0; base < chunk_hits; base += 4 * 32) {  // warp-uniform
       const uint32_t j0 = base + lane;
@@ -307,7 +334,7 @@ __global__ void __launch_bounds__(WPB * 32) consolidate_fit_kernel(ChainPointers
         const uint32_t j = p0 + lane;
         const uint32_t t = started + __popc(heads & (0xFFFFFFFFu >> (31 - lane))) - 1;  // track of j
         started += __popc(heads);
-        hh[u] = j < chunk_hits ? track_hits[(i0 + t) * kMaxTrackSize + (j - s_off[warp][t])] : 0u;
+        hh[u] = j < chunk_hits ? track_hits[(i0 + t) * kMaxTrackSize + (chunk0 + j - s_off[i0 + t])] : 0u;
       }
       float4 p[4];
       uint32_t id[4];
@@ -336,11 +363,10 @@ __global__ void __launch_bounds__(WPB * 32) consolidate_fit_kernel(ChainPointers
     }
     __syncwarp();
     if (i < nt) {
-      const uint32_t hoff = carry + s_off[warp][lane];
-      P.track_hit_number[t0 + i] = hoff;
+      const uint32_t o = s_off[i] - chunk0, n = s_off[i + 1] - s_off[i];
+      P.track_hit_number[t0 + i] = carry + o;
       FitState beam, kal;
       if (staged) {
-        const uint32_t o = s_off[warp][lane];
         beam = beamline_fit(&s_hit[warp][0][o], &s_hit[warp][1][o], &s_hit[warp][2][o], n);
         kal = kalman_fit(&s_hit[warp][0][o], &s_hit[warp][1][o], &s_hit[warp][2][o], n, beam);
       } else {
@@ -357,7 +383,6 @@ __global__ void __launch_bounds__(WPB * 32) consolidate_fit_kernel(ChainPointers
       store_state(P.states, T, t0 + i, beam);
       store_state(P.kalman_states, T, t0 + i, kal);
     }
-    carry += chunk_hits;
     __syncwarp();
   }
 }
