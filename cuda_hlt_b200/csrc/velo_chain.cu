@@ -362,7 +362,7 @@ int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaS
   VCK(cudaGetLastError());
   ++c->launches;
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][4], s, capturing));
-  consolidate_fit_kernel<4><<<(n + 3) / 4, 128, 0, s>>>(P);
+  consolidate_fit_kernel<kConsolidateWarps><<<n, kConsolidateWarps * 32, 0, s>>>(P);
   VCK(cudaGetLastError());
   ++c->launches;
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][5], s, capturing));
