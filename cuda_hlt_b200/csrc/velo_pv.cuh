@@ -5,9 +5,9 @@
 //   1. every track is extrapolated to its point of closest approach to the beamline
 //      (pv_beamline_extrapolate.cu:3-30, the PVTrack constructor of
 //      TrackBeamLineVertexFinder.cuh:9-31) into a scratch array;
-//   2. the z histogram (2400 bins of 0.25 mm) lives in shared memory only: each warp owns a
-//      quarter of the bins and adds every track's contributions to them, tracks in order, a
-//      track's bins over the lanes. The reference adds with float atomics into global memory
+//   2. the z histogram (2400 bins of 0.25 mm) lives in shared memory only: each thread works out
+//      one track's window, then each warp, which owns a quarter of the bins, adds the tracks
+//      that reach into it, in order, a track's bins over the lanes. The reference adds with float atomics into global memory
 //      (pv_beamline_histo.cu:14-76), so its bins carry an arbitrary summation order; these
 //      are reproducible. Each bin receives the same per-track contributions,
 //      G(bin) - G(bin - 1) of the polynomial Gaussian integral G;
@@ -87,9 +87,9 @@ __device__ __forceinline__ float pv_gauss_integral(float x)
 // Contribution of a track to bin i of its window [minbin, maxbin]: the difference of the
 // integral at the bin's upper edge and at the previous bin's (0 before the first bin; the
 // last bin receives the rest up to 1).
-__device__ __forceinline__ float pv_bin_contribution(const PvTrack& t, float zerr, int minbin, int maxbin, int i)
+__device__ __forceinline__ float pv_bin_contribution(float z, float zerr, int minbin, int maxbin, int i)
 {
-  auto g = [&](int b) { return pv_gauss_integral((kPvZmin + (b + 1) * kPvDz - t.z) / zerr); };
+  auto g = [&](int b) { return pv_gauss_integral((kPvZmin + (b + 1) * kPvDz - z) / zerr); };
   const float below = i > minbin ? g(i - 1) : 0.f;
   return (i < maxbin ? g(i) : 1.f) - below;
 }
@@ -103,8 +103,15 @@ constexpr uint32_t kPvMaxToggles = 512;  // changes between empty and filled bin
 
 constexpr int kPvBinsPerWarp = kPvBins / kPvWarps;
 
+// A track's histogram window [minbin, maxbin], empty when the track is not used.
+struct PvWindow {
+  float z, zerr;
+  int minbin, maxbin;
+};
+
 struct PvSmem {
   float histo[kPvBins];
+  PvWindow window[kPvThreads];
   float zpeaks[kPvMaxVertices];
   uint32_t n_peaks, flags;
   uint16_t tog[kPvMaxToggles];
@@ -117,9 +124,9 @@ struct PvSmem {
 __global__ void __launch_bounds__(kPvThreads) pv_beamline_kernel(ChainPointers P, PvPointers V)
 {
   __shared__ PvSmem s;
-  const uint32_t e = blockIdx.x;
   const uint32_t N = P.run->n_events;
-  if (e >= N) return;
+  if (blockIdx.x >= N) return;
+  const uint32_t e = P.event_order[blockIdx.x];  // largest first
   const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
   const uint32_t T = P.atomics[2 * N];
   const uint32_t nt = P.atomics[e];
@@ -156,24 +163,46 @@ __global__ void __launch_bounds__(kPvThreads) pv_beamline_kernel(ChainPointers P
   __syncthreads();
 
   // ---- 2. z histogram: warp w fills bins [w * 600, (w + 1) * 600) from every track, in order ----
+  // (each warp working out every track's window itself, a chain of a load, two square roots and
+  // three quotients a track, took the stage 0.459 ms for 4,096 events; so 0.327)
   {
     float* h = s.histo;
     const int own_lo = static_cast<int>(warp) * kPvBinsPerWarp, own_hi = own_lo + kPvBinsPerWarp - 1;
-    for (uint32_t i = 0; i < nt; ++i) {
-      const PvTrack t = tracks[i];
-      if (!(kPvZmin < t.z && t.z < kPvZmax)) continue;
-      const float zbin = (t.z - kPvZmin) / kPvDz;
-      const float zweight = t.tx * t.tx * t.w00 + t.ty * t.ty * t.w11;
-      const float zerr = 1.f / sqrtf(zweight);
-      if (!(zerr < kPvMaxTrackZ0Err)) continue;
-      const float a = sqrtf(float(2 * kPvOrderPolynomial + 3));
-      const float halfwindow = a * zerr / kPvDz;
-      const int minbin = max(int(zbin - halfwindow), 1);
-      const int maxbin = min(int(zbin + halfwindow), kPvBins - 2);
-      const int first = max(minbin, own_lo), last = min(maxbin, own_hi);
-      for (int b = first + static_cast<int>(lane); b <= last; b += 32)
-        h[b] += pv_bin_contribution(t, zerr, minbin, maxbin, b);
-      __syncwarp();
+    for (uint32_t i0 = 0; i0 < nt; i0 += kPvThreads) {
+      PvWindow w{0.f, 0.f, 1, 0};
+      if (i0 + threadIdx.x < nt) {
+        const PvTrack t = tracks[i0 + threadIdx.x];  // written by this thread
+        if (kPvZmin < t.z && t.z < kPvZmax) {
+          const float zbin = (t.z - kPvZmin) / kPvDz;
+          const float zweight = t.tx * t.tx * t.w00 + t.ty * t.ty * t.w11;
+          const float zerr = 1.f / sqrtf(zweight);
+          if (zerr < kPvMaxTrackZ0Err) {
+            const float a = sqrtf(float(2 * kPvOrderPolynomial + 3));
+            const float halfwindow = a * zerr / kPvDz;
+            w.z = t.z;
+            w.zerr = zerr;
+            w.minbin = max(int(zbin - halfwindow), 1);
+            w.maxbin = min(int(zbin + halfwindow), kPvBins - 2);
+          }
+        }
+      }
+      __syncthreads();  // the windows before have been added
+      s.window[threadIdx.x] = w;
+      __syncthreads();
+      for (uint32_t g = 0; g < kPvThreads && i0 + g < nt; g += 32) {
+        const PvWindow mine = s.window[g + lane];
+        // the tracks of this group with bins in this warp's quarter
+        uint32_t todo = __ballot_sync(0xFFFFFFFFu, mine.minbin <= mine.maxbin && mine.minbin <= own_hi &&
+                                                     mine.maxbin >= own_lo);
+        while (todo) {
+          const PvWindow t = s.window[g + __ffs(todo) - 1];
+          todo &= todo - 1;
+          const int first = max(t.minbin, own_lo), last = min(t.maxbin, own_hi);
+          for (int b = first + static_cast<int>(lane); b <= last; b += 32)
+            h[b] += pv_bin_contribution(t.z, t.zerr, t.minbin, t.maxbin, b);
+          __syncwarp();
+        }
+      }
     }
   }
   __syncthreads();
