@@ -77,6 +77,7 @@ struct VeloCtx {
   char *d_track_hits_out = nullptr, *d_states = nullptr, *d_kalman = nullptr;
   uint32_t* d_queue = nullptr;
   uint32_t* d_event_order = nullptr;
+  ulonglong2* d_scan_sums = nullptr;
   uint32_t block_threshold = 0;  // clusters above which an event takes the block search
   // beamline PV stage (velo_set_pv)
   bool pv = false;
@@ -166,7 +167,7 @@ void free_all(VeloCtx* c)
                   c->d_event_hits, c->d_status, c->d_track_n, c->d_track_hits, c->d_tracklets, c->d_weak, c->d_ttf,
                   c->d_event_tracks, c->d_event_track_hits, c->d_atomics, c->d_track_hit_number,
                   c->d_event_hit_offset, c->d_track_hits_out, c->d_states, c->d_kalman, c->d_queue,
-                  c->d_event_order, c->d_pv_tracks, c->d_pv_vertices,
+                  c->d_event_order, c->d_scan_sums, c->d_pv_tracks, c->d_pv_vertices,
                   c->d_pv_count, c->d_pv_npeaks, c->d_pv_zpeaks, c->d_gec_counts, c->d_event_list,
                   c->d_n_selected, c->d_gec_flags, c->d_gec_ut, c->d_gec_scifi, c->d_gec_ut_offsets,
                   c->d_gec_scifi_offsets};
@@ -230,6 +231,8 @@ ChainPointers pointers(VeloCtx* c, uint32_t n_grid)
   P.track_hits_out = c->d_track_hits_out;
   P.states = c->d_states;
   P.kalman_states = c->d_kalman;
+  P.scan_sums = c->d_scan_sums;
+  P.totals = c->h_totals;
   P.max_tracks_total = c->cfg.max_tracks;
   P.max_track_hits_total = c->cfg.max_track_hits;
   P.hit_capacity = c->hit_capacity;
@@ -358,9 +361,18 @@ int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaS
     c->launches += 2;
   }
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][3], s, capturing));
-  event_scan_kernel<<<1, 1024, 0, s>>>(P);
-  VCK(cudaGetLastError());
-  ++c->launches;
+  if (n <= kScanOneBlock) {
+    event_scan_kernel<<<1, 1024, 0, s>>>(P);
+    VCK(cudaGetLastError());
+    ++c->launches;
+  } else {
+    const uint32_t blocks = (n + kScanBlock - 1) / kScanBlock;
+    event_sum_kernel<<<blocks, kScanBlock, 0, s>>>(P);
+    VCK(cudaGetLastError());
+    event_scan_blocks_kernel<<<blocks, kScanBlock, 0, s>>>(P);
+    VCK(cudaGetLastError());
+    c->launches += 2;
+  }
   if (c->timing && c->ev_current >= 0) VCK(record(c->ev_sets[c->ev_current][4], s, capturing));
   consolidate_fit_kernel<kConsolidateWarps><<<n, kConsolidateWarps * 32, 0, s>>>(P);
   VCK(cudaGetLastError());
@@ -531,6 +543,7 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   ok &= dalloc(c->d_gec_scifi_offsets, static_cast<size_t>(N) + 1) == cudaSuccess;
   ok &= dalloc(c->d_queue, 8) == cudaSuccess;
   ok &= dalloc(c->d_event_order, N) == cudaSuccess;
+  ok &= dalloc(c->d_scan_sums, static_cast<size_t>(N) / kScanBlock + 1) == cudaSuccess;
   ok &= cudaMallocHost(reinterpret_cast<void**>(&c->h_totals), 4 * sizeof(uint32_t) + 8) == cudaSuccess;
   ok &= cudaMallocHost(reinterpret_cast<void**>(&c->h_offsets), 3 * (static_cast<size_t>(N) + 1) * sizeof(uint64_t)) ==
         cudaSuccess;
@@ -733,24 +746,18 @@ static int launch_run(VeloCtx* c, const void* raw, const uint64_t* raw_offsets, 
   return rc;
 }
 
-// Reads the run's totals (tracks, track hits, error bits) into the pinned h_totals on the
-// run's stream, queued right behind the run so that velo_sync only waits: a read queued at
-// sync time would wait behind whatever the caller queued on the stream's copy engine since.
-static int queue_totals(VeloCtx* c, cudaStream_t s, uint32_t n)
-{
-  VCK(cudaMemcpyAsync(c->h_totals, c->d_atomics + 2 * n, 4, cudaMemcpyDeviceToHost, s));
-  VCK(cudaMemcpyAsync(c->h_totals + 1, c->d_event_hit_offset + n, 4, cudaMemcpyDeviceToHost, s));
-  VCK(cudaMemcpyAsync(c->h_totals + 2, c->d_queue + 6, 4, cudaMemcpyDeviceToHost, s));
-  return 0;
-}
-
 static int run_chain(VeloCtx* c, const void* raw, const uint64_t* raw_offsets, const uint32_t* raw_offsets32,
                      const VeloGecInput* gec, uint32_t n_events, void* stream, VeloOutputs* out,
                      const uint32_t* event_list = nullptr, uint32_t n_raw = 0)
 {
   const int rc = launch_run(c, raw, raw_offsets, raw_offsets32, gec, n_events, stream, out, event_list, n_raw);
-  if (rc) return rc;
-  return queue_totals(c, static_cast<cudaStream_t>(stream), n_events);
+  if (rc || n_events) return rc;  // the scan wrote the run's totals to h_totals
+  // an empty batch launches no kernel: its zeros follow the earlier runs on the stream
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  VCK(cudaMemcpyAsync(c->h_totals, c->d_atomics, 4, cudaMemcpyDeviceToHost, s));
+  VCK(cudaMemcpyAsync(c->h_totals + 1, c->d_event_hit_offset, 4, cudaMemcpyDeviceToHost, s));
+  VCK(cudaMemcpyAsync(c->h_totals + 2, c->d_queue + 6, 4, cudaMemcpyDeviceToHost, s));
+  return 0;
 }
 
 int velo_run(VeloCtx* c, const void* raw, const uint64_t* raw_offsets, uint32_t n_events, void* stream,

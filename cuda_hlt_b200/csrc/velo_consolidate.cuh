@@ -6,9 +6,20 @@
 
 namespace velo {
 
-// Exclusive scans of tracks and track hits per event (single block), in the layout of
-// copy_and_prefix_sum_single_block + the track-hit prefix sum (PrefixSumSingleBlock.cu:130-168).
-__global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
+// The run's totals, where velo_sync reads them: pinned host memory, written by the kernel that
+// knows them, so no copy follows the run.
+__device__ __forceinline__ void store_totals(const ChainPointers& P, uint32_t tracks, uint32_t hits)
+{
+  P.totals[0] = tracks;
+  P.totals[1] = hits;
+  P.totals[2] = P.queue[6];
+}
+
+// Exclusive scans of tracks and track hits per event by one block of 1024 threads, in the
+// layout of copy_and_prefix_sum_single_block + the track-hit prefix sum
+// (PrefixSumSingleBlock.cu:130-168). An event beyond the consolidated output capacity keeps no
+// tracks.
+__device__ __forceinline__ void scan_events_one_block(const ChainPointers& P)
 {
   __shared__ uint32_t s_warp_t[32], s_warp_h[32];
   const uint32_t N = P.run->n_events;
@@ -72,9 +83,102 @@ __global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
     P.atomics[2 * N] = ot;
     P.event_hit_offset[N] = oh;
     P.track_hit_number[ot] = oh;
+    store_totals(P, ot, oh);
   }
 }
 
+__global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
+{
+  scan_events_one_block(P);
+}
+
+// The same scans for batches of more than kScanOneBlock events, kScanBlock events a block in two
+// launches: one block walks a thread's run of events one after the other, at uncoalesced
+// addresses, and takes 4.8 us per 1,000 events (65,536: 0.315 ms, so 0.014). A batch that exceeds
+// the output capacity goes through the one block, whose rule for what is dropped holds then.
+constexpr uint32_t kScanBlock = 1024;
+constexpr uint32_t kScanOneBlock = 4096;
+
+// Sum over the block of x and y; s_sum: 32 entries.
+__device__ __forceinline__ ulonglong2 scan_block_sum(unsigned long long x, unsigned long long y, ulonglong2* s_sum)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+    y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
+  }
+  __syncthreads();
+  if (lane_id() == 0) s_sum[threadIdx.x >> 5] = make_ulonglong2(x, y);
+  __syncthreads();
+  ulonglong2 t = s_sum[lane_id()];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t.x += __shfl_xor_sync(0xFFFFFFFFu, t.x, o);
+    t.y += __shfl_xor_sync(0xFFFFFFFFu, t.y, o);
+  }
+  return t;
+}
+
+__global__ void __launch_bounds__(kScanBlock) event_sum_kernel(ChainPointers P)
+{
+  __shared__ ulonglong2 s_sum[32];
+  const uint32_t e = blockIdx.x * kScanBlock + threadIdx.x;
+  const bool in = e < P.run->n_events;
+  const ulonglong2 t = scan_block_sum(in ? P.event_tracks[e] : 0u, in ? P.event_track_hits[e] : 0u, s_sum);
+  if (threadIdx.x == 0) P.scan_sums[blockIdx.x] = t;
+}
+
+__global__ void __launch_bounds__(kScanBlock) event_scan_blocks_kernel(ChainPointers P)
+{
+  __shared__ ulonglong2 s_sum[32];
+  __shared__ uint2 s_warp[32];
+  const uint32_t N = P.run->n_events, lane = lane_id(), warp = threadIdx.x >> 5;
+  // sums of the blocks before this one, and of all
+  unsigned long long bt = 0, bh = 0, at = 0, ah = 0;
+  for (uint32_t b = threadIdx.x; b < gridDim.x; b += kScanBlock) {
+    const ulonglong2 v = P.scan_sums[b];
+    at += v.x;
+    ah += v.y;
+    if (b < blockIdx.x) {
+      bt += v.x;
+      bh += v.y;
+    }
+  }
+  const ulonglong2 all = scan_block_sum(at, ah, s_sum), before = scan_block_sum(bt, bh, s_sum);
+  if (all.x > P.max_tracks_total || all.y > P.max_track_hits_total) {
+    if (blockIdx.x == 0) scan_events_one_block(P);
+    return;
+  }
+  const uint32_t e = blockIdx.x * kScanBlock + threadIdx.x;
+  const uint32_t t = e < N ? P.event_tracks[e] : 0u, h = e < N ? P.event_track_hits[e] : 0u;
+  uint32_t it = t, ih = h;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t vt = __shfl_up_sync(0xFFFFFFFFu, it, o), vh = __shfl_up_sync(0xFFFFFFFFu, ih, o);
+    if (lane >= static_cast<uint32_t>(o)) {
+      it += vt;
+      ih += vh;
+    }
+  }
+  if (lane == 31) s_warp[warp] = make_uint2(it, ih);
+  __syncthreads();
+  uint32_t wt = static_cast<uint32_t>(before.x), wh = static_cast<uint32_t>(before.y);
+  for (uint32_t w = 0; w < warp; ++w) {
+    wt += s_warp[w].x;
+    wh += s_warp[w].y;
+  }
+  if (e < N) {
+    P.atomics[e] = t;
+    P.atomics[N + e] = wt + it - t;
+    P.event_hit_offset[e] = wh + ih - h;
+    if (e == N - 1) {
+      P.atomics[2 * N] = wt + it;
+      P.event_hit_offset[N] = wh + ih;
+      P.track_hit_number[wt + it] = wh + ih;
+      store_totals(P, wt + it, wh + ih);
+    }
+  }
+}
 
 struct FitState {
   float x, y, tx, ty, c00, c20, c22, c11, c31, c33, chi2, z;

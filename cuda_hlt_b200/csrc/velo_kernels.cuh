@@ -134,6 +134,8 @@ struct ChainPointers {
   char* track_hits_out;
   char* states;
   char* kalman_states;
+  ulonglong2* scan_sums;       // [N / 1024 + 1] tracks and track hits of each 1,024 events
+  uint32_t* totals;            // [4] pinned host memory: tracks, track hits, error bits of the run
   uint32_t max_tracks_total;
   uint32_t max_track_hits_total;
   uint64_t hit_capacity;       // entries of the hit SoA arrays
