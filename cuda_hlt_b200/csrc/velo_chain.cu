@@ -71,7 +71,7 @@ struct VeloCtx {
   uint32_t *d_module_start = nullptr, *d_module_num = nullptr, *d_event_hit_base = nullptr, *d_event_hits = nullptr,
            *d_status = nullptr;
   uint16_t *d_track_n = nullptr, *d_track_hits = nullptr, *d_tracklets = nullptr, *d_weak = nullptr;
-  uint32_t* d_ttf = nullptr;
+  uint2* d_ttf = nullptr;
   uint32_t *d_event_tracks = nullptr, *d_event_track_hits = nullptr;
   uint32_t *d_atomics = nullptr, *d_track_hit_number = nullptr, *d_event_hit_offset = nullptr;
   char *d_track_hits_out = nullptr, *d_states = nullptr, *d_kalman = nullptr;

@@ -69,7 +69,7 @@ struct SearchScratch {
   uint16_t* track_n;       // [N * kMaxTracks]
   uint16_t* track_hits;    // [N * kMaxTracks * kMaxTrackSize]
   uint16_t* tracklets;     // [N * kTrackletRing * 3]
-  uint32_t* ttf;           // [N * kTtfModulo]
+  uint2* ttf;              // [N * kTtfModulo]
   uint16_t* weak;          // [N * kWeakCap * 3]
 };
 

@@ -477,7 +477,7 @@ struct EventScratch {
   uint16_t* track_n;     // [kMaxTracks]
   uint16_t* track_hits;  // [kMaxTracks * kMaxTrackSize]
   uint16_t* tracklets;   // [kTrackletRing * 3]
-  uint32_t* ttf;         // [kTtfModulo]
+  uint2* ttf;            // [kTtfModulo] {track and state bits, last hit << 16 | the hit before}
   uint16_t* weak;        // [kWeakCap * 3]
 };
 
@@ -545,7 +545,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
   uint16_t* track_n = sc.track_n;
   uint16_t* track_hits = sc.track_hits;
   uint16_t* tracklets = sc.tracklets;
-  uint32_t* ttf = sc.ttf;
+  uint2* ttf = sc.ttf;
   uint16_t* weak = sc.weak;
   uint32_t n_tracks = 0, tracklet_ptr = 0, ttf_ptr = 0, weak_ptr = 0;
   uint32_t last_seeded = 0;
@@ -613,10 +613,11 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
           const unsigned long long key = sl.best[k];
           if (static_cast<uint32_t>(key >> 32) == sl.tie[k]) flags |= kStatusSeedTie;
           const uint32_t tp = (tracklet_ptr + rank) % kTrackletRing;
-          tracklets[3 * tp] = static_cast<uint16_t>(sl.f0[k] + ((key >> 16) & 0xFFFFu));
-          tracklets[3 * tp + 1] = sl.h1[k];
-          tracklets[3 * tp + 2] = static_cast<uint16_t>(sl.f2[k] + (key & 0xFFFFu));
-          ttf[(ttf_ptr + rank) % kTtfModulo] = 0x80000000u | tp;
+          const uint32_t h1 = sl.h1[k], h2 = sl.f2[k] + (static_cast<uint32_t>(key) & 0xFFFFu);
+          tracklets[3 * tp] = static_cast<uint16_t>(sl.f0[k] + (static_cast<uint32_t>(key) >> 16));
+          tracklets[3 * tp + 1] = static_cast<uint16_t>(h1);
+          tracklets[3 * tp + 2] = static_cast<uint16_t>(h2);
+          ttf[(ttf_ptr + rank) % kTtfModulo] = make_uint2(0x80000000u | tp, (h2 << 16) | h1);
         }
         at += nwin;
       }
@@ -702,28 +703,25 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     for (uint32_t i0 = 0; i0 < diff; i0 += 32 * G) {
       const uint32_t i = i0 + tid;
       int action = 0;  // 1 extend, 2 keep with a skipped module, 3 demote to weak
-      uint32_t full = 0, trackno = 0, nhit = 0;
-      uint16_t t0 = 0, t1 = 0, t2 = 0, best_h2 = 0;
+      uint32_t full = 0, last_two = 0, trackno = 0, nhit = 0;
+      uint16_t t0 = 0, best_h2 = 0;
       if (i < diff) {
-        full = ttf[(prev_ttf + i) % kTtfModulo];
-        const bool flag = (full & 0x80000000u) == 0x80000000u;
+        // the entry brings the hits the prediction needs, two dependent loads fewer than through
+        // the track (search of 65,536 events 13.18 -> 12.81 ms, of 1,000 0.271 -> 0.255); what
+        // only an extension needs follows
+        const uint2 entry = ttf[(prev_ttf + i) % kTtfModulo];
+        full = entry.x;
+        last_two = entry.y;
+        const float4 h0 = H[last_two & 0xFFFFu];
+        const float4 h1 = H[last_two >> 16];
         const uint32_t skipped = (full & 0x70000000u) >> 28;
         trackno = full & 0x0FFFFFFFu;
-        uint16_t ha, hb;
-        if (flag) {
+        if (full & 0x80000000u) {
           t0 = tracklets[3 * trackno];
-          t1 = tracklets[3 * trackno + 1];
-          t2 = tracklets[3 * trackno + 2];
           nhit = 3;
-          ha = t1;
-          hb = t2;
         } else {
           nhit = track_n[trackno];
-          ha = track_hits[trackno * kMaxTrackSize + nhit - 2];
-          hb = track_hits[trackno * kMaxTrackSize + nhit - 1];
         }
-        const float4 h0 = H[ha];
-        const float4 h1 = H[hb];
         const float td = 1.0f / (h1.z - h0.z);
         const float txn = (h1.x - h0.x);
         const float tyn = (h1.y - h0.y);
@@ -743,8 +741,8 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
         set_used(used, best_h2);
         if (nhit == 3) {
           set_used(used, t0);
-          set_used(used, t1);
-          set_used(used, t2);
+          set_used(used, last_two & 0xFFFFu);
+          set_used(used, last_two >> 16);
         }
       }
       const bool is_new = action == 1 && nhit == 3;
@@ -760,8 +758,8 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
         if (slot < kMaxTracks) {
           uint16_t* th = track_hits + slot * kMaxTrackSize;
           th[0] = t0;
-          th[1] = t1;
-          th[2] = t2;
+          th[1] = static_cast<uint16_t>(last_two);
+          th[2] = static_cast<uint16_t>(last_two >> 16);
           th[3] = best_h2;
           track_n[slot] = 4;
           trackno = slot;
@@ -775,16 +773,16 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
       if (all_dropped) flags |= kStatusTrackOverflow;
       n_tracks = all_tracks - all_dropped;
       if (stored || action == 2) {
-        const uint32_t value =
-          action == 2 ? ((((full & 0x70000000u) >> 28) + 1) << 28) | (full & 0x8FFFFFFFu) : trackno;
-        ttf[(ttf_ptr + rank[1] - dropped) % kTtfModulo] = value;
+        ttf[(ttf_ptr + rank[1] - dropped) % kTtfModulo] =
+          action == 2 ? make_uint2(((((full & 0x70000000u) >> 28) + 1) << 28) | (full & 0x8FFFFFFFu), last_two)
+                      : make_uint2(trackno, (last_two >> 16) | (static_cast<uint32_t>(best_h2) << 16));
       }
       ttf_ptr += total[1] - all_dropped;
       if (action == 3 && weak_ptr + rank[2] < kWeakCap) {
         uint16_t* w = weak + 3 * (weak_ptr + rank[2]);
         w[0] = t0;
-        w[1] = t1;
-        w[2] = t2;
+        w[1] = static_cast<uint16_t>(last_two);
+        w[2] = static_cast<uint16_t>(last_two >> 16);
       }
       weak_ptr += total[2];
     }
@@ -812,7 +810,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     for (uint32_t i0 = 0; i0 < diff; i0 += 32 * G) {
       const uint32_t i = i0 + tid;
       uint32_t full = 0;
-      if (i < diff) full = ttf[(prev + i) % kTtfModulo];
+      if (i < diff) full = ttf[(prev + i) % kTtfModulo].x;
       const bool is_weak = i < diff && (full & 0x80000000u);
       uint32_t rank[3], total[3];
       group_rank<G>(sh, turn, is_weak, false, false, rank, total);

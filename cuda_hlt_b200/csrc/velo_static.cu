@@ -28,11 +28,11 @@ namespace {
 
 constexpr uint32_t kStaticMaxEvents = 512;
 constexpr size_t kTrackletBytes = kTrackletRing * 3 * sizeof(uint16_t);  // 12000
-constexpr size_t kTtfBytes = kTtfModulo * sizeof(uint32_t);                // 8000
+constexpr size_t kTtfBytes = kTtfModulo * sizeof(uint2);                   // 16000
 constexpr size_t kWeakBytes = kWeakCap * 3 * sizeof(uint16_t);            // 24576
 constexpr size_t kEventScratchBytes = ((kTrackletBytes + kTtfBytes + kWeakBytes + 255) / 256) * 256;
 constexpr size_t kStaticHeaderBytes = 256;  // work-queue counter, zeroed by every call
-constexpr size_t kStaticScratchBytes = kStaticHeaderBytes + kStaticMaxEvents * kEventScratchBytes;  // ~22.9 MB
+constexpr size_t kStaticScratchBytes = kStaticHeaderBytes + kStaticMaxEvents * kEventScratchBytes;  // ~27.0 MB
 
 // The scratch. In host code this name is only a stand-in for the device symbol: kernels get
 // the device address looked up by cudaGetSymbolAddress below.
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(128) search_static_kernel(StaticSearchArgs A)
       const EventScratch sc{A.track_n + static_cast<size_t>(e) * kMaxTracks,
                             A.track_hits + static_cast<size_t>(e) * kMaxTracks * kMaxTrackSize,
                             reinterpret_cast<uint16_t*>(ev_scratch),
-                            reinterpret_cast<uint32_t*>(ev_scratch + kTrackletBytes),
+                            reinterpret_cast<uint2*>(ev_scratch + kTrackletBytes),
                             reinterpret_cast<uint16_t*>(ev_scratch + kTrackletBytes + kTtfBytes)};
       n_tracks = search_event<1>(sw, H, ComputedWindows{H, sw.mstart, sw.mnum}, nullptr, sc, flags);
     }

@@ -426,7 +426,7 @@ int velo_graph_count(VeloCtx* ctx, uint32_t* n);
  * velo_run (VeloOutputs hit_xyzp, module_hit_start, module_hit_num, status) and writes the
  * tracks of each event in the reference's Velo::TrackHits terms: track_n[n * 1200] hit
  * counts and track_hits[n * 1200 * 26] event-relative hit indices, event_tracks[n] and
- * status_out[n]. Its scratch is a fixed ~23 MB __device__ array, resident on every device
+ * status_out[n]. Its scratch is a fixed ~27 MB __device__ array, resident on every device
  * that loads the library: at most 512 events per call (more: VELO_ERR_CAPACITY), all calls
  * share it (calls overlapping on a device race), and the first call on a device looks up
  * its address, so that first call should come before any stream capture. Calls no
