@@ -162,7 +162,7 @@ __device__ __forceinline__ bool flood_window(uint32_t px0, uint32_t px1, uint32_
 }
 
 constexpr uint32_t kCandCap = 4096;    // candidate pixels listed per event (more: flooded inline)
-constexpr uint32_t kBankMapCap = 16384; // SPs per event with a bank map (more: binary search)
+constexpr uint32_t kNoCandidate = 0xFFFFFFFFu;  // (bank 255 does not exist)
 constexpr uint32_t kNonIsoCap = 2048;   // non-isolated SPs listed per event (more: full rescan)
 constexpr uint32_t kRegSortMax = 256;  // modules up to this size are sorted in registers
 
@@ -174,6 +174,7 @@ struct DecodeShared {
   uint32_t unsorted[(kSensors + 31) / 32];
   uint32_t mod_count[kModules];  // clusters per module
   uint32_t mod_start[kModules];  // exclusive scan of mod_count: compact layout
+  uint32_t mod_phi[kModules];    // exclusive scan over the modules of the same parity
   uint32_t event;
   uint32_t n_events;             // events of the run
   uint32_t skipped;              // 1: position left empty (beyond the selection); 2: bad list entry
@@ -199,13 +200,7 @@ struct DecodeEvent {
   uint32_t stage_base;      // first staging slot of the event
   float4* stage;
   uint32_t* stage_id;
-  const uint8_t* bank_map;  // bank of each flat SP index (shared memory), or null
 };
-
-__device__ __forceinline__ uint32_t bank_of_sp(const DecodeShared& sh, const DecodeEvent& d, uint32_t f)
-{
-  return d.bank_map ? d.bank_map[f] : bank_of(sh, f);
-}
 
 // Bits 26-27 of an LHCb VP id are always zero (sensor < 208 ends at bit 25): the staging
 // record carries the cluster's pixel count there, at most 3.
@@ -224,12 +219,11 @@ __device__ __forceinline__ void stage_cluster(DecodeShared& sh, const DecodeEven
   d.stage_id[o] = p.id | (min(pixels, 3u) << kSizeShift);
 }
 
-// Flood fill of candidate pixel k of flat SP f and staging of the cluster
+// Flood fill of candidate pixel k of flat SP f, of bank b, and staging of the cluster
 // (MaskedVeloClustering.cu:175-461).
 __device__ __forceinline__ void flood_candidate(DecodeShared& sh, const DecodeEvent& d, const GeometryView& g,
-                                                uint32_t f, uint32_t k)
+                                                uint32_t f, uint32_t b, uint32_t k)
 {
-  const uint32_t b = bank_of_sp(sh, d, f);
   const uint32_t s = f - sh.sp_prefix[b];
   const uint32_t* bank = d.ev + sh.bank_start[b];
   const uint32_t count = sh.bank_count[b];
@@ -377,22 +371,19 @@ __device__ __forceinline__ void warp_smem_sort(unsigned long long* key, uint32_t
   }
 }
 
-// Shared-memory capacity for the event's phi in the windows pass (the union below, free once
-// the modules are sorted); larger events search their windows in the cluster records.
-constexpr uint32_t kPhiStageCap = (kCandCap * 4 + kBankMapCap + kNonIsoCap * 2) / 4;
-
 // Phi windows of the h1 of one module, after the event's modules are sorted
 // (fill_candidates, FillCandidates.cu:8-70, VeloTools.cuh:6-42): for each hit h1 of module m
 // (2..49) the hits within kPhiExtrapolation of phi(h1) in module m + 2 (h0) and m - 2 (h2),
-// as event-relative u16 pairs {first | last << 16} (0xFFFF: none). `sphi` holds the event's
-// phi in hit order (null: read the cluster records). In the pruned mode also the scorer's
+// as event-relative u16 pairs {first | last << 16} (0xFFFF: none). `sphi` holds the modules'
+// phi, module m's from mphi[m] on (null: read the cluster records). In the pruned mode also the scorer's
 // inputs: keep bits (3: seeding candidate, verdict to come; 2: no seed) and, for each
 // candidate the gates admit, an 8-byte record (event hit base, h1 | m << 16) appended to the
 // candidate list (queue slot 7). One warp per module; every lane takes part in each 32-hit
 // round (ballots). Bound by the integer pipe: the branch-free searches took decode of 65,536
 // events at nu ~ U(2,20) from 11.24 to 10.80 ms.
 template<bool kPruned>
-__device__ __forceinline__ void module_windows(const ChainPointers& P, const float* sphi, const float4* H, uint2* Wn,
+__device__ __forceinline__ void module_windows(const ChainPointers& P, const float* sphi, const uint32_t* mphi,
+                                               const float4* H, uint2* Wn,
                                                uint8_t* K, uint32_t base, uint32_t m, const uint32_t* mstart,
                                                const uint32_t* mcount, bool score)
 {
@@ -406,9 +397,9 @@ __device__ __forceinline__ void module_windows(const ChainPointers& P, const flo
     int f0 = -1, l0 = -1, f2 = -1, l2 = -1;
     if (valid) {
       if (sphi) {
-        const float p = sphi[h];
-        if (n0 > 0) phi_window_flat(sphi + s0, n0, p, kPhiExtrapolation, f0, l0);
-        if (n2 > 0) phi_window_flat(sphi + s2, n2, p, kPhiExtrapolation, f2, l2);
+        const float p = sphi[mphi[m] + r];
+        if (n0 > 0) phi_window_flat(sphi + mphi[m + 2], n0, p, kPhiExtrapolation, f0, l0);
+        if (n2 > 0) phi_window_flat(sphi + mphi[m - 2], n2, p, kPhiExtrapolation, f2, l2);
         if (f0 != -1) {
           f0 += s0;
           l0 += s0;
@@ -448,9 +439,8 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
   // the candidate list and the per-warp sort buffers are never live together
   __shared__ union {
     struct {
-      uint32_t cand[kCandCap];
-      uint8_t bank_map[kBankMapCap];  // flat SP index -> bank, saves a binary search per SP
-      uint16_t noniso[kNonIsoCap];    // flat SP indices of the non-isolated SPs
+      uint32_t cand[kCandCap];      // flat SP index << 12 | bank << 4 | pixel
+      uint32_t noniso[kNonIsoCap];  // non-isolated SPs: bank << 16 | flat SP index
     } lists;
     unsigned long long key[W][kSortCap];
   } su;
@@ -547,10 +537,8 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
     __syncthreads();
     const uint32_t total_sp = sh.sp_prefix[kSensors];
     const uint32_t base = static_cast<uint32_t>(off / 4);
-    const bool use_map = event_ok && total_sp <= kBankMapCap;  // counts are valid only then
-    const DecodeEvent d{ev, 2 * base, P.stage.xyzp, P.stage.id, use_map ? su.lists.bank_map : nullptr};
-    // ---- pass 1, one pass over the flat SP index: bank of every SP (map), sortedness of each
-    // bank, and the clusters of the isolated SPs from the pattern table (they need neither);
+    const DecodeEvent d{ev, 2 * base, P.stage.xyzp, P.stage.id};
+    // ---- pass 1, one pass over the flat SP index: the sortedness of each bank, and the clusters of the isolated SPs from the pattern table (they need neither);
     // the non-isolated SPs are listed for pass 2. Every thread's loads are independent, so
     // the first touches of the raw event overlap instead of queueing bank by bank ----
     const bool can_list = total_sp <= 0x10000u;  // list entries are 16-bit
@@ -562,7 +550,6 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
       uint32_t b = warp * run < f_end ? bank_of(sh, warp * run) : 0u;
       for (uint32_t f = warp * run + lane; f < f_end; f += 32) {
         while (sh.sp_prefix[b + 1] <= f) ++b;
-        if (use_map) su.lists.bank_map[f] = static_cast<uint8_t>(b);
         const uint32_t s = f - sh.sp_prefix[b];
         const uint32_t* bank = ev + sh.bank_start[b];
         const uint32_t word = __ldg(bank + s);
@@ -587,7 +574,7 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
           }
         } else if (can_list) {
           const uint32_t q = atomicAdd(&sh.n_noniso, 1u);
-          if (q < kNonIsoCap) su.lists.noniso[q] = static_cast<uint16_t>(f);
+          if (q < kNonIsoCap) su.lists.noniso[q] = (b << 16) | f;
         }
       }
     }
@@ -598,8 +585,8 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
     const bool listed = can_list && sh.n_noniso <= kNonIsoCap;
     const uint32_t n_scan = listed ? sh.n_noniso : total_sp;
     for (uint32_t i = threadIdx.x; i < n_scan; i += blockDim.x) {
-      const uint32_t f = listed ? su.lists.noniso[i] : i;
-      const uint32_t b = bank_of_sp(sh, d, f);
+      const uint32_t f = listed ? su.lists.noniso[i] & 0xFFFFu : i;
+      const uint32_t b = listed ? su.lists.noniso[i] >> 16 : bank_of(sh, f);
       const uint32_t s = f - sh.sp_prefix[b];
       const uint32_t* bank = ev + sh.bank_start[b];
       const uint32_t word = __ldg(bank + s);
@@ -614,8 +601,11 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
         ++my_cands;
         const uint32_t k = candidate_k(nib) + 2 * half;
         const uint32_t slot = atomicAdd(&sh.n_list, 1u);
-        if (slot < kCandCap) su.lists.cand[slot] = (f << 4) | k;
-        else flood_candidate(sh, d, g, f, k);
+        if (slot < kCandCap && f < (1u << 20)) su.lists.cand[slot] = (f << 12) | (b << 4) | k;
+        else {
+          if (slot < kCandCap) su.lists.cand[slot] = kNoCandidate;
+          flood_candidate(sh, d, g, f, b, k);
+        }
       }
     }
 #pragma unroll
@@ -626,7 +616,7 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
     const uint32_t n_list = min(sh.n_list, kCandCap);
     for (uint32_t i = threadIdx.x; i < n_list; i += blockDim.x) {
       const uint32_t c = su.lists.cand[i];
-      flood_candidate(sh, d, g, c >> 4, c & 0xFu);
+      if (c != kNoCandidate) flood_candidate(sh, d, g, c >> 12, (c >> 4) & 0xFFu, c & 0xFu);
     }
     __syncthreads();
     // ---- compact layout: exclusive scan of the module counts ----
@@ -709,10 +699,18 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
       const uint32_t nh = write ? sh.mod_start[kModules - 1] + sh.mod_count[kModules - 1] : 0;
       if (nh > 0 && nh <= kEventHitCap) {  // the events the search runs
         const float4* H = P.hits.xyzp + base;
-        float* sphi = nh <= kPhiStageCap ? reinterpret_cast<float*>(&su) : nullptr;
-        if (sphi)
-          for (uint32_t i = threadIdx.x; i < nh; i += blockDim.x) sphi[i] = H[i].w;
-        __syncthreads();
+        // A window joins modules of one parity, so an event whose phi do not fit the shared
+        // memory takes the even modules first, then the odd ones; what does not fit then either
+        // searches the cluster records.
+        constexpr uint32_t kPhiCap = sizeof(su) / sizeof(float);
+        const bool whole = nh <= kPhiCap;
+        if (!whole && threadIdx.x < 2) {
+          uint32_t n = 0;
+          for (uint32_t m = threadIdx.x; m < kModules; m += 2) {
+            sh.mod_phi[m] = n;
+            n += sh.mod_count[m];
+          }
+        }
         bool score = false;
         uint8_t* K = nullptr;
         if (kPruned) {
@@ -730,17 +728,32 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
             for (uint32_t h = threadIdx.x; h < nh; h += blockDim.x) K[h] = 3;
           }
         }
-        bool scored = false;
-        if constexpr (kPruned) {
-          if (score) {
-            for (uint32_t m = 2 + warp; m < 50; m += W)
-              module_windows<true>(P, sphi, H, P.windows + base, K, base, m, sh.mod_start, sh.mod_count, true);
-            scored = true;
+        for (uint32_t half = 0; half < (whole ? 1u : 2u); ++half) {
+          float* sphi = reinterpret_cast<float*>(&su);
+          const uint32_t* mphi = whole ? sh.mod_start : sh.mod_phi;
+          __syncthreads();  // mod_phi written; the half before searched
+          if (whole) {
+            for (uint32_t i = threadIdx.x; i < nh; i += blockDim.x) sphi[i] = H[i].w;
+          } else if (mphi[kModules - 2 + half] + sh.mod_count[kModules - 2 + half] <= kPhiCap) {
+            for (uint32_t m = half + 2 * warp; m < kModules; m += 2 * W)
+              for (uint32_t i = lane; i < sh.mod_count[m]; i += 32) sphi[mphi[m] + i] = H[sh.mod_start[m] + i].w;
+          } else {
+            sphi = nullptr;
           }
+          __syncthreads();
+          const uint32_t first = 2 + (whole ? warp : half + 2 * warp), step = whole ? W : 2 * W;
+          bool scored = false;
+          if constexpr (kPruned) {
+            if (score) {
+              for (uint32_t m = first; m < 50; m += step)
+                module_windows<true>(P, sphi, mphi, H, P.windows + base, K, base, m, sh.mod_start, sh.mod_count, true);
+              scored = true;
+            }
+          }
+          if (!scored)
+            for (uint32_t m = first; m < 50; m += step)
+              module_windows<false>(P, sphi, mphi, H, P.windows + base, K, base, m, sh.mod_start, sh.mod_count, false);
         }
-        if (!scored)
-          for (uint32_t m = 2 + warp; m < 50; m += W)
-            module_windows<false>(P, sphi, H, P.windows + base, K, base, m, sh.mod_start, sh.mod_count, false);
       }
     }
     __syncthreads();
