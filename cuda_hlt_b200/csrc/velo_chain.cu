@@ -34,11 +34,9 @@ struct VeloCtx {
   int sm_count = 0;
   cudaStream_t own_stream = nullptr;
   // constants
-  uint8_t* d_geometry = nullptr;
-  uint8_t* d_sp_patterns = nullptr;
-  float* d_sp_fx = nullptr;
-  float* d_sp_fy = nullptr;
-  uint8_t* d_sp_sizes = nullptr;
+  float4* d_ltg = nullptr;
+  float2* d_local_x = nullptr;
+  SpCluster* d_sp = nullptr;
   // learned scorer
   __nv_bfloat16* d_mlp_w = nullptr;
   float* d_mlp_norm = nullptr;
@@ -161,7 +159,7 @@ cudaError_t dalloc(T*& p, size_t count)
 
 void free_all(VeloCtx* c)
 {
-  void* ptrs[] = {c->d_labels, c->d_geometry, c->d_sp_patterns, c->d_sp_fx, c->d_sp_fy, c->d_sp_sizes, c->d_mlp_w, c->d_mlp_norm,
+  void* ptrs[] = {c->d_labels, c->d_ltg, c->d_local_x, c->d_sp, c->d_mlp_w, c->d_mlp_norm,
                   c->d_hit_size, c->d_windows, c->d_keep, c->d_cand_slot, c->d_cand_rec, c->d_raw, c->d_raw_offsets, c->d_hxyzp,
                   c->d_hid, c->d_stage_xyzp, c->d_stage_id, c->d_module_start, c->d_module_num, c->d_event_hit_base,
                   c->d_event_hits, c->d_status, c->d_track_n, c->d_track_hits, c->d_tracklets, c->d_weak, c->d_ttf,
@@ -207,8 +205,7 @@ ChainPointers pointers(VeloCtx* c, uint32_t n_grid)
   ChainPointers P{};
   P.run = c->d_run;
   P.n_grid = n_grid;
-  P.k = DeviceConstants{reinterpret_cast<const float*>(c->d_geometry), c->d_sp_patterns, c->d_sp_fx, c->d_sp_fy,
-                        c->d_sp_sizes};
+  P.k = DeviceConstants{c->d_ltg, c->d_local_x, c->d_sp};
   P.hits = HitsAoS{c->d_hxyzp, c->d_hid};
   P.stage = HitsAoS{c->d_stage_xyzp, c->d_stage_id};
   P.module_start = c->d_module_start;
@@ -310,6 +307,12 @@ cudaError_t record(cudaEvent_t e, cudaStream_t s, bool capturing)
   return capturing ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
 }
 
+template<int W, bool kPruned>
+void launch_decode(const ChainPointers& P, uint32_t blocks, cudaStream_t s)
+{
+  decode_cluster_sort_kernel<W, kPruned><<<blocks, W * 32, sizeof(DecodeLists<W>), s>>>(P);
+}
+
 int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaStream_t s, bool capturing = false)
 {
   const uint32_t n = P.n_grid;
@@ -330,12 +333,16 @@ int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaS
     const uint32_t blocks = std::min<uint32_t>(n, c->decode_blocks);
     // the decode kernel also computes the phi windows (fill_candidates) and, in the pruned
     // mode, the scorer's candidate list
-    if (c->decode_warps == 8) {
-      if (pruned) decode_cluster_sort_kernel<8, true><<<blocks, 256, 0, s>>>(P);
-      else decode_cluster_sort_kernel<8, false><<<blocks, 256, 0, s>>>(P);
+    const int warps = c->decode_warps == 8 && n <= kDecodeWide * c->sm_count ? 16 : c->decode_warps;
+    if (warps == 16) {
+      if (pruned) launch_decode<16, true>(P, blocks, s);
+      else launch_decode<16, false>(P, blocks, s);
+    } else if (warps == 8) {
+      if (pruned) launch_decode<8, true>(P, blocks, s);
+      else launch_decode<8, false>(P, blocks, s);
     } else {
-      if (pruned) decode_cluster_sort_kernel<4, true><<<blocks, 128, 0, s>>>(P);
-      else decode_cluster_sort_kernel<4, false><<<blocks, 128, 0, s>>>(P);
+      if (pruned) launch_decode<4, true>(P, blocks, s);
+      else launch_decode<4, false>(P, blocks, s);
     }
     VCK(cudaGetLastError());
     ++c->launches;
@@ -393,9 +400,9 @@ void size_decode_grid(VeloCtx* c)
 {
   int occ = 0;
   if (c->decode_warps == 8)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_cluster_sort_kernel<8, true>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_cluster_sort_kernel<8, true>, 256, sizeof(DecodeLists<8>));
   else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_cluster_sort_kernel<4, true>, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, decode_cluster_sort_kernel<4, true>, 128, sizeof(DecodeLists<4>));
   c->decode_blocks = static_cast<uint32_t>(std::max(1, occ) * c->sm_count);
 }
 
@@ -493,11 +500,9 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   c->hit_capacity = cfg->max_raw_bytes / 4 + 64;
   const size_t T = c->cfg.max_tracks, TH = c->cfg.max_track_hits;
   bool ok = true;
-  ok &= dalloc(c->d_geometry, kGeometryBytes) == cudaSuccess;
-  ok &= dalloc(c->d_sp_patterns, 256) == cudaSuccess;
-  ok &= dalloc(c->d_sp_fx, 512) == cudaSuccess;
-  ok &= dalloc(c->d_sp_fy, 512) == cudaSuccess;
-  ok &= dalloc(c->d_sp_sizes, 256) == cudaSuccess;
+  ok &= dalloc(c->d_ltg, kSensors * 4) == cudaSuccess;
+  ok &= dalloc(c->d_local_x, kPixelColumns) == cudaSuccess;
+  ok &= dalloc(c->d_sp, 512) == cudaSuccess;
   ok &= dalloc(c->d_mlp_w, kMlpParams) == cudaSuccess;
   ok &= dalloc(c->d_mlp_norm, 32) == cudaSuccess;
   ok &= dalloc(c->d_raw, cfg->max_raw_bytes + 16) == cudaSuccess;
@@ -553,13 +558,27 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   uint8_t pat[256], sizes[256];
   float fx[512], fy[512];
   velo_build_sp_luts(pat, sizes, fx, fy);
-  if (cudaMemcpy(c->d_geometry, geometry, kGeometryBytes, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(c->d_sp_patterns, pat, 256, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(c->d_sp_fx, fx, sizeof fx, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(c->d_sp_fy, fy, sizeof fy, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(c->d_sp_sizes, sizes, 256, cudaMemcpyHostToDevice) != cudaSuccess)
+  std::vector<SpCluster> sp(512);
+  for (int m = 0; m < 256; ++m)
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t row = k ? (pat[m] >> 4) & 3u : pat[m] & 3u, col = k ? (pat[m] >> 6) & 1u : (pat[m] >> 2) & 1u;
+      const uint32_t more = k == 0 && (pat[m] & 8u) ? 8u : 0u;
+      sp[2 * m + k] = SpCluster{fx[2 * m + k], fy[2 * m + k],
+                                row | col << 2 | more | static_cast<uint32_t>((sizes[m] >> (4 * k)) & 0xF) << 4, 0u};
+    }
+  std::vector<float> blob(kGeometryBytes / 4);  // the caller's may stand at any address
+  std::memcpy(blob.data(), geometry, kGeometryBytes);
+  std::vector<float2> column(kPixelColumns);
+  for (uint32_t i = 0; i < kPixelColumns; ++i) column[i] = make_float2(blob[i], blob[kSensorColumns + i]);
+  if (cudaMemcpy(c->d_ltg, blob.data() + 2 * kSensorColumns, kSensors * 64, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(c->d_local_x, column.data(), column.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(c->d_sp, sp.data(), sp.size() * sizeof(SpCluster), cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(VELO_ERR_CUDA);
   int occ = 0;
+  cudaFuncSetAttribute(decode_cluster_sort_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       sizeof(DecodeLists<16>));
+  cudaFuncSetAttribute(decode_cluster_sort_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       sizeof(DecodeLists<16>));
   size_decode_grid(c);
   size_search_grid(c);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gec_count_kernel, kGecThreads, 0);

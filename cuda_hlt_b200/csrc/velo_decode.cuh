@@ -221,7 +221,7 @@ __device__ __forceinline__ void stage_cluster(DecodeShared& sh, const DecodeEven
 
 // Flood fill of candidate pixel k of flat SP f, of bank b, and staging of the cluster
 // (MaskedVeloClustering.cu:175-461).
-__device__ __forceinline__ void flood_candidate(DecodeShared& sh, const DecodeEvent& d, const GeometryView& g,
+__device__ __forceinline__ void flood_candidate(DecodeShared& sh, const DecodeEvent& d, const DeviceConstants& g,
                                                 uint32_t f, uint32_t b, uint32_t k)
 {
   const uint32_t s = f - sh.sp_prefix[b];
@@ -430,22 +430,31 @@ __device__ __forceinline__ void module_windows(const ChainPointers& P, const flo
   }
 }
 
-// 40 warps per SM (5 blocks of 8): 48 registers, no spills. kPruned: the windows pass also
-// prepares the learned scorer's candidate list.
+// The block's lists, then its sort buffers (one a warp), then the event's phi: never live
+// together. Dynamic shared memory: 16 warps need 64 KB.
+template<int W>
+union DecodeLists {
+  struct {
+    uint32_t cand[kCandCap];      // flat SP index << 12 | bank << 4 | pixel
+    uint32_t noniso[kNonIsoCap];  // non-isolated SPs: bank << 16 | flat SP index
+  } lists;
+  unsigned long long key[W][kSortCap];
+};
+
+// 40 warps per SM (5 blocks of 8): 48 registers, no spills (6 blocks at 40 registers: 10.5
+// instead of 10.0 ms for 65,536 events). Bound by the integer pipe and issue; a batch of at most
+// kDecodeWide events per SM, which leaves the device idle, takes 16 warps an event (10 events at
+// nu ~ U(2,15) 92 -> 60 us, 148 100 -> 66, 290 133 -> 90; two such blocks fill an SM). kPruned:
+// the windows pass also prepares the learned scorer's candidate list.
+constexpr uint32_t kDecodeWide = 2;
+
 template<int W, bool kPruned>
 __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(ChainPointers P)
 {
   __shared__ DecodeShared sh;
-  // the candidate list and the per-warp sort buffers are never live together
-  __shared__ union {
-    struct {
-      uint32_t cand[kCandCap];      // flat SP index << 12 | bank << 4 | pixel
-      uint32_t noniso[kNonIsoCap];  // non-isolated SPs: bank << 16 | flat SP index
-    } lists;
-    unsigned long long key[W][kSortCap];
-  } su;
+  extern __shared__ __align__(16) uint8_t s_dyn[];
+  DecodeLists<W>& su = *reinterpret_cast<DecodeLists<W>*>(s_dyn);
   const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
-  const GeometryView g = geometry_view(P.k.geometry);
 
   for (;;) {
     if (threadIdx.x == 0) {
@@ -558,19 +567,16 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
           // pattern table (MaskedVeloClustering.cu:105-167)
           const uint32_t sp = sp_mask(word);
           const int32_t sp_r = sp_row(word), sp_c = sp_col(word);
-          const uint32_t idx = __ldg(P.k.sp_patterns + sp);
           const uint32_t chip = sp_c / (kChipColumns / 2);
           const uint32_t sensor = sh.bank_sensor[b];
           for (int c = 0; c < 2; ++c) {
-            if (c == 1 && !(idx & 8)) break;
-            const uint32_t row = c ? (idx >> 4) & 3u : idx & 0x03u;
-            const uint32_t col = c ? (idx >> 6) & 1u : (idx >> 2) & 1u;
-            const uint32_t cx = sp_c * 2 + col;
-            const uint32_t cy = sp_r * 4 + row;
-            const float fx = __ldg(P.k.sp_fx + sp * 2 + c);
-            const float fy = __ldg(P.k.sp_fy + sp * 2 + c);
-            stage_cluster(sh, d, b >> 2, place_cluster(g, sensor, cx, cy, fx, fy, chip),
-                          (__ldg(P.k.sp_sizes + sp) >> (4 * c)) & 0xFu);
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(P.k.sp + 2 * sp + c));
+            const uint32_t cx = sp_c * 2 + ((v.z >> 2) & 1u);
+            const uint32_t cy = sp_r * 4 + (v.z & 3u);
+            stage_cluster(sh, d, b >> 2,
+                          place_cluster(P.k, sensor, cx, cy, __uint_as_float(v.x), __uint_as_float(v.y), chip),
+                          (v.z >> 4) & 0xFu);
+            if (!(v.z & 8u)) break;
           }
         } else if (can_list) {
           const uint32_t q = atomicAdd(&sh.n_noniso, 1u);
@@ -604,7 +610,7 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
         if (slot < kCandCap && f < (1u << 20)) su.lists.cand[slot] = (f << 12) | (b << 4) | k;
         else {
           if (slot < kCandCap) su.lists.cand[slot] = kNoCandidate;
-          flood_candidate(sh, d, g, f, b, k);
+          flood_candidate(sh, d, P.k, f, b, k);
         }
       }
     }
@@ -616,7 +622,7 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
     const uint32_t n_list = min(sh.n_list, kCandCap);
     for (uint32_t i = threadIdx.x; i < n_list; i += blockDim.x) {
       const uint32_t c = su.lists.cand[i];
-      if (c != kNoCandidate) flood_candidate(sh, d, g, c >> 12, (c >> 4) & 0xFFu, c & 0xFu);
+      if (c != kNoCandidate) flood_candidate(sh, d, P.k, c >> 12, (c >> 4) & 0xFFu, c & 0xFu);
     }
     __syncthreads();
     // ---- compact layout: exclusive scan of the module counts ----
@@ -702,7 +708,7 @@ __global__ void __launch_bounds__(W * 32, 40 / W) decode_cluster_sort_kernel(Cha
         // A window joins modules of one parity, so an event whose phi do not fit the shared
         // memory takes the even modules first, then the odd ones; what does not fit then either
         // searches the cluster records.
-        constexpr uint32_t kPhiCap = sizeof(su) / sizeof(float);
+        constexpr uint32_t kPhiCap = sizeof(DecodeLists<W>) / sizeof(float);
         const bool whole = nh <= kPhiCap;
         if (!whole && threadIdx.x < 2) {
           uint32_t n = 0;

@@ -37,12 +37,22 @@ constexpr uint32_t kStatusSeedTie = 1u << 11;           // exact scatter tie in 
 
 __constant__ float c_module_z[kModules] = {VELO_MODULE_Z_VALUES};
 
+// One of the (up to two) clusters of an isolated SP, by its pixel pattern: one 16-byte load in
+// the place of one per table of cache_sp_patterns (ClusteringCommon.cpp:3-101).
+struct SpCluster {
+  float fx, fy;   // fraction of a pixel
+  uint32_t info;  // bits 0-1 row, 2 column, 3 a second cluster follows, 4-7 pixels
+  uint32_t pad;
+};
+
+// Pixel columns that an SP word can name (9 bits of SP column, two pixels each): beyond the
+// sensor's 768 the table holds what stands there in the blob, as a read past its columns would.
+constexpr uint32_t kPixelColumns = 1024;
+
 struct DeviceConstants {
-  const float* geometry;      // 19456-byte blob
-  const uint8_t* sp_patterns; // [256]
-  const float* sp_fx;         // [512]
-  const float* sp_fy;         // [512]
-  const uint8_t* sp_sizes;    // [256] pixels of the first (low nibble) and second cluster
+  const float4* ltg;           // [208 * 4] sensor to global: the geometry blob's 16 floats a sensor
+  const float2* local_x;       // [kPixelColumns] {local_x, x_pitch} of the geometry blob
+  const SpCluster* sp;         // [256 * 2]
 };
 
 // Parameters of the learned seed/extension scorer as the kernels read them.
@@ -191,16 +201,20 @@ struct ClusterPoint {
   uint32_t id;
 };
 
-__device__ __forceinline__ ClusterPoint place_cluster(const GeometryView& g, uint32_t sensor, uint32_t cx, uint32_t cy,
-                                                      float fx, float fy, uint32_t chip)
+__device__ __forceinline__ ClusterPoint place_cluster(const DeviceConstants& k, uint32_t sensor, uint32_t cx,
+                                                      uint32_t cy, float fx, float fy, uint32_t chip)
 {
-  const float* ltg = g.ltg + 16 * sensor;
-  const float local_x = g.local_x[cx] + fx * g.x_pitch[cx];
+  const float4* ltg = k.ltg + 4 * sensor;  // floats 0 .. 11 of the sensor's 16
+  const float4 a = __ldg(ltg), b = __ldg(ltg + 1), c = __ldg(ltg + 2);
+  const float2 column = __ldg(k.local_x + cx);
+  const float local_x = __fmaf_rn(fx, column.y, column.x);
   const float local_y = (cy + 0.5 + fy) * kPixelSize;
+  // the reference's sums as its build contracts them, written out: how the compiler contracts
+  // the plain expressions depends on the loads around them
   ClusterPoint p;
-  p.x = ltg[0] * local_x + ltg[1] * local_y + ltg[9];
-  p.y = ltg[3] * local_x + ltg[4] * local_y + ltg[10];
-  p.z = ltg[6] * local_x + ltg[7] * local_y + ltg[11];
+  p.x = __fadd_rn(__fmaf_rn(a.x, local_x, __fmul_rn(a.y, local_y)), c.y);
+  p.y = __fadd_rn(__fmaf_rn(a.w, local_x, __fmul_rn(b.x, local_y)), c.z);
+  p.z = __fadd_rn(__fmaf_rn(b.z, local_x, __fmul_rn(b.w, local_y)), c.w);
   p.id = lhcb_id(channel_id(sensor, chip, cx % kChipColumns, cy));
   return p;
 }

@@ -403,8 +403,9 @@ int velo_set_pv(VeloCtx* ctx, int enabled);
  * (cuda_hlt_b200/autotune.py) from timings per hit-count bucket. */
 int velo_set_block_threshold(VeloCtx* ctx, uint32_t clusters);
 
-/* Decode block size: 4 or 8 warps per event (default 8); set by the autotuner
- * (cuda_hlt_b200/autotune.py) from decode timings on a sample batch. */
+/* Decode block size: 4 or 8 warps per event (default 8, of which a batch of at most two events
+ * per SM makes 16); set by the autotuner (cuda_hlt_b200/autotune.py) from decode timings on a
+ * sample batch. */
 int velo_set_decode_warps(VeloCtx* ctx, uint32_t warps);
 
 /* Diagnostics of the error path of the bounded device waits: runs one kernel that waits, for
