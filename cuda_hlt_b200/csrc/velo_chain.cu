@@ -362,8 +362,10 @@ int launch_chain(VeloCtx* c, const ChainPointers& P, const GecPointers* G, cudaS
   {
     order_events_kernel<<<1, kOrderThreads, 0, s>>>(P);
     VCK(cudaGetLastError());
-    // at least a block for each event that might take one
-    search_kernel<kSearchWarps><<<std::min<uint32_t>(n, c->search_blocks), kSearchWarps * 32, 0, s>>>(P);
+    if (n <= kSmallBatch * c->sm_count)
+      search_kernel<kSmallBatchWarps><<<n, kSmallBatchWarps * 32, 0, s>>>(P);
+    else  // at least a block for each event that might take one
+      search_kernel<kSearchWarps><<<std::min<uint32_t>(n, c->search_blocks), kSearchWarps * 32, 0, s>>>(P);
     VCK(cudaGetLastError());
     c->launches += 2;
   }

@@ -327,16 +327,37 @@ __device__ __forceinline__ void seed_flush(SeedSlots& sl, uint32_t nc, const flo
   __syncwarp();
 }
 
-// Shared state of one event searched by G warps. Forwarding reads the phi of its two target
-// modules from shared memory, one after the other in a staging area that reuses the seeding
-// slots (the two phases never overlap).
+// Eight warps an event are for a batch too small to fill the device (kSmallBatch): the steps are
+// chains of dependent loads with most warps waiting at the barriers, so what a step will read is
+// fetched during the one before. In a full device the extra loads (the windows of used h1, the
+// copies' instructions) cost more than they hide: four warps an event with it took 1.90 ms for
+// 3,000 noisy events, 1.73 without.
+template<int G>
+constexpr bool kFetchAhead = G >= 8;
+
+// The phi of the two modules that forwarding searches, one after the other in shared memory: in
+// a staging area that reuses the seeding slots (the two phases never overlap), so that L1 keeps
+// its share of the SM, or in one of its own where it is filled during the seeding.
+template<int G, bool kAhead = kFetchAhead<G>>
+union SeedArea {
+  static constexpr uint32_t kFwdStage = G * sizeof(SeedSlots) / sizeof(float);
+  SeedSlots seed[G];  // one per warp
+  float fphi[kFwdStage];
+};
+template<int G>
+union SeedArea<G, true> {
+  static constexpr uint32_t kFwdStage = 2048;
+  struct {
+    SeedSlots seed[G];
+    float fphi[kFwdStage];
+  };
+};
+
+// Shared state of one event searched by G warps.
 template<int G>
 struct SearchShared {
-  static constexpr uint32_t kFwdStage = G * sizeof(SeedSlots) / sizeof(float);
-  union {
-    SeedSlots seed[G];  // one per warp
-    float fphi[kFwdStage];
-  } u;
+  static constexpr uint32_t kFwdStage = SeedArea<G>::kFwdStage;
+  SeedArea<G> u;
   uint32_t used[kEventHitCap / 32];
   uint32_t mstart[kModules];
   uint32_t mnum[kModules];
@@ -351,6 +372,16 @@ __device__ __forceinline__ uint32_t group_thread()
 {
   return G == 1 ? lane_id() : threadIdx.x;
 }
+// Asynchronous copy of one float from global to shared memory; a thread's copies are complete
+// after async_wait.
+__device__ __forceinline__ void async_copy4(float* dst, const float* src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template<int G>
 __device__ __forceinline__ void group_sync()
 {
@@ -551,6 +582,28 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
   uint32_t last_seeded = 0;
   uint32_t turn = 0;
 
+  // Ahead of their step: the phi of the forwarding's modules (stage) and the windows of the
+  // seeding's first run (fetch).
+  auto stage = [&](uint32_t first) {
+    const uint32_t mo = first - 4, me = first - 5, mon = mnum[mo], men = mnum[me];
+    if (mon + men > SearchShared<G>::kFwdStage) return;
+    const float4 *Ho = H + mstart[mo], *He = H + mstart[me];
+    for (uint32_t i = tid; i < mon; i += 32 * G) async_copy4(&sh.u.fphi[i], &Ho[i].w);
+    for (uint32_t i = tid; i < men; i += 32 * G) async_copy4(&sh.u.fphi[mon + i], &He[i].w);
+  };
+  uint2 fetched[kSeedChunk / 32];
+  auto fetch = [&](uint32_t first) {
+    const uint32_t ma = first - 2, mb = first - 3, na = mnum[ma], n_list = na + mnum[mb];
+    const uint32_t run = (min(n_list, G * kSeedChunk) + G - 1) / G;
+    const uint32_t lo = min(n_list, warp * run), hi = min(n_list, lo + run);
+#pragma unroll
+    for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
+      const uint32_t r = lo + 32 * j + lane;
+      fetched[j] = make_uint2(0xFFFFu, 0xFFFFu);
+      if (r < hi) fetched[j] = r < na ? windows(mstart[ma] + r, ma) : windows(mstart[mb] + r - na, mb);
+    }
+  };
+
   // ---- seeding: h1 in modules first-2 / first-3, h0 in h1+2, h2 in h1-2 ----
   // The two modules' seeds are independent (seeding marks no hit used). One warp takes the
   // modules' h1 in turn (first - 2, then first - 3), queueing unused ones with windows until
@@ -566,13 +619,16 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     // the next (up to) kSeedChunk h1, hit_of(r) for r in [r0, r_end): unused, with both phi
     // windows (FillCandidates.cu:31-68, TrackSeeding.cu:24-49); the windows of their 32-hit
     // groups are loaded together so that their latencies overlap
-    auto gather = [&](uint32_t r0, uint32_t r_end, auto hit_of, auto module_of) {
+    auto gather = [&](uint32_t r0, uint32_t r_end, auto hit_of, auto module_of, bool have_windows) {
       uint32_t n_new = 0;
 #pragma unroll
       for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
         const uint32_t r = r0 + 32 * j + lane;
         wv[j] = make_uint2(0xFFFFu, 0xFFFFu);
-        if (r < r_end && !test_used(used, hit_of(r))) wv[j] = windows(hit_of(r), module_of(r));
+        if (r < r_end && !test_used(used, hit_of(r))) {
+          if constexpr (kFetchAhead<G>) wv[j] = have_windows ? fetched[j] : windows(hit_of(r), module_of(r));
+          else wv[j] = windows(hit_of(r), module_of(r));
+        }
       }
 #pragma unroll
       for (uint32_t j = 0; j < kSeedChunk / 32; ++j) {
@@ -637,7 +693,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
         const uint32_t m = first - (have ? side : 3);
         const uint32_t start = mstart[m];
         auto hit_of = [&](uint32_t r) { return start + r; };
-        const uint32_t n_new = gather(r0, have ? min(mnum[m], r0 + kSeedChunk) : 0u, hit_of, [&](uint32_t) { return m; });
+        const uint32_t n_new = gather(r0, have ? min(mnum[m], r0 + kSeedChunk) : 0u, hit_of, [&](uint32_t) { return m; }, false);
         if (nc > 0 && (!have || nc + n_new > kSeedChunk)) {
           seed_flush(sl, nc, H, used);
           const uint32_t n = append(0);
@@ -656,7 +712,8 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
       for (uint32_t r0 = 0; r0 < n_list; r0 += G * kSeedChunk) {
         const uint32_t run = (min(n_list - r0, G * kSeedChunk) + G - 1) / G;
         const uint32_t lo = min(n_list, r0 + warp * run), hi = min(n_list, lo + run);
-        const uint32_t n_new = gather(lo, hi, hit_of, [&](uint32_t r) { return r < na ? ma : mb; });
+        const uint32_t n_new = gather(lo, hi, hit_of, [&](uint32_t r) { return r < na ? ma : mb; },
+                                      kFetchAhead<G> && r0 == 0);
         queue(lo, hit_of);
         if (nc > 0) seed_flush(sl, nc, H, used);
         uint32_t nwin = 0;
@@ -690,12 +747,14 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     const uint32_t mo = first - 4, me = first - 5;
     const uint32_t mos = mstart[mo], mon = mnum[mo], mes = mstart[me], men = mnum[me];
     const float moz = c_module_z[mo], mez = c_module_z[me];
-    // stage the phi of both target modules (their searches then stay in shared memory); a pair
-    // of modules above the staging size is searched in global memory
+    // the phi of both target modules in shared memory, where their searches stay; a pair of
+    // modules above the staging size is searched in global memory
     const bool fits = mon + men <= SearchShared<G>::kFwdStage;
     const float* sphi_o = fits ? sh.u.fphi : nullptr;
     const float* sphi_e = fits ? sh.u.fphi + mon : nullptr;
-    if (diff > 0 && fits) {
+    if constexpr (kFetchAhead<G>) {
+      async_wait();  // staged during the seeding before
+    } else if (diff > 0 && fits) {
       for (uint32_t i = tid; i < mon; i += 32 * G) sh.u.fphi[i] = H[mos + i].w;
       for (uint32_t i = tid; i < men; i += 32 * G) sh.u.fphi[mon + i] = H[mes + i].w;
     }
@@ -791,6 +850,10 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
 
   // ---- module loop (ProcessModules.cu:37-162) ----
   uint32_t first = kModules - 1;
+  if constexpr (kFetchAhead<G>) {
+    fetch(first);
+    stage(first - 2);
+  }
   seeding(first);
   uint32_t last_ttf = 0;
   first -= 2;
@@ -798,8 +861,11 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     const uint32_t prev = last_ttf;
     last_ttf = ttf_ptr;
     if (last_ttf - prev > kTtfModulo) flags |= kStatusTtfOverflow;
+    if constexpr (kFetchAhead<G>) fetch(first);
     forwarding(first, prev, last_ttf - prev);
     if (ttf_ptr - prev > kTtfModulo) flags |= kStatusTtfOverflow;
+    if constexpr (kFetchAhead<G>)
+      if (first >= 6) stage(first - 2);
     seeding(first);
     first -= 2;
   }
@@ -914,6 +980,13 @@ __device__ __forceinline__ void search_chain_event(SearchShared<G>& sh, const Ch
 // 8 blocks of 4 warps per SM at 64 registers: more resident events (10 or 12 blocks at 48 or
 // 40 registers) measured slower, their hit records competing for L1.
 constexpr int kSearchWarps = 4;
+
+// A batch of at most kSmallBatch events per SM takes eight warps an event, all of them resident
+// at once: search of 10 / 148 / 300 / 590 events at nu ~ U(2,15) 0.251 / 0.273 / 0.325 / 0.398 ms
+// with four, 0.183 / 0.185 / 0.221 / 0.287 with eight. Beyond one wave the uneven batches still
+// gain (1,000 events 0.44 -> 0.39), the even ones lose (1,000 at nu = 7.6 0.26 -> 0.32).
+constexpr int kSmallBatchWarps = 8;
+constexpr uint32_t kSmallBatch = 4;
 
 template<int W>
 __global__ void __launch_bounds__(W * 32, 32 / W) search_kernel(ChainPointers P)
