@@ -75,23 +75,33 @@ constexpr uint32_t kScoreSmem = sizeof(ScoreSmem) + 128;
 __device__ __forceinline__ uint32_t score_half() { return threadIdx.x >> 7; }
 __device__ __forceinline__ uint32_t score_row() { return threadIdx.x & (kMlpTile - 1); }
 
+// ReLU of two accumulators in bf16: rounded, then cut at zero in one packed instruction (the
+// same values as cut first).
+__device__ __forceinline__ uint32_t relu_bf16x2(float a, float b)
+{
+  const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(a, b), __nv_bfloat162(__float2bfloat16_rn(0.f), __float2bfloat16_rn(0.f)));
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // Epilogue of a hidden layer for this thread's row: ReLU of the 64 accumulators, rounded to
 // bf16 into columns 0..63 of the row of H (the ones column stays).
 __device__ __forceinline__ void score_hidden_epilogue(uint8_t* h, uint32_t taddr_row, uint32_t row)
 {
 #pragma unroll
-  for (uint32_t c = 0; c < 4; ++c) {
-    float v[16];
-    tmem_ld16(taddr_row + 16 * c, v);
+  for (uint32_t c = 0; c < 2; ++c) {
+    float v[2][16];
+    tmem_ld16(taddr_row + 32 * c, v[0]);
+    tmem_ld16(taddr_row + 32 * c + 16, v[1]);
     tmem_ld_wait();
 #pragma unroll
-    for (uint32_t u = 0; u < 2; ++u) {
+    for (uint32_t u = 0; u < 4; ++u) {
+      const float* w = v[u >> 1] + 8 * (u & 1);
       uint4 q;
-      q.x = pack_bf16x2(fmaxf(v[8 * u + 0], 0.f), fmaxf(v[8 * u + 1], 0.f));
-      q.y = pack_bf16x2(fmaxf(v[8 * u + 2], 0.f), fmaxf(v[8 * u + 3], 0.f));
-      q.z = pack_bf16x2(fmaxf(v[8 * u + 4], 0.f), fmaxf(v[8 * u + 5], 0.f));
-      q.w = pack_bf16x2(fmaxf(v[8 * u + 6], 0.f), fmaxf(v[8 * u + 7], 0.f));
-      *reinterpret_cast<uint4*>(h + canon_off(row, 2 * c + u, kSbo2)) = q;
+      q.x = relu_bf16x2(w[0], w[1]);
+      q.y = relu_bf16x2(w[2], w[3]);
+      q.z = relu_bf16x2(w[4], w[5]);
+      q.w = relu_bf16x2(w[6], w[7]);
+      *reinterpret_cast<uint4*>(h + canon_off(row, 4 * c + u, kSbo2)) = q;
     }
   }
 }

@@ -361,17 +361,28 @@ __device__ __forceinline__ bool mlp_tile_forward(MlpInferSmem& s, uint32_t& phas
 // ---------------------------------------------------------------------------------
 // Features of the proxy triplet of h1
 // ---------------------------------------------------------------------------------
-// The hits of window [f, l) of a phi-sorted module that bracket phi1: the last with
-// phi < phi1 and the first with phi >= phi1 (one of them when phi1 is outside the window).
-__device__ __forceinline__ void bracket(const float4* H, int f, int l, float phi1, int& a, int& b)
+// The hits of the windows [f0, l0) and [f2, l2) of two phi-sorted modules that bracket phi1: the
+// last with phi < phi1 and the first with phi >= phi1 (one of them when phi1 is outside the
+// window). Each probe is a load that the next one waits for, so the two searches step together.
+__device__ __forceinline__ void bracket_pair(const float4* H, int f0, int l0, int f2, int l2, float phi1, int (&c0)[2],
+                                             int (&c2)[2])
 {
-  int lo = f, hi = l;  // first index in [f, l) with phi >= phi1
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (H[mid].w < phi1) lo = mid + 1; else hi = mid;
+  int lo0 = f0, hi0 = l0, lo2 = f2, hi2 = l2;  // first index in [f, l) with phi >= phi1
+  while (lo0 < hi0 || lo2 < hi2) {
+    const int mid0 = (lo0 + hi0) >> 1, mid2 = (lo2 + hi2) >> 1;
+    const bool on0 = lo0 < hi0, on2 = lo2 < hi2;
+    const float p0 = on0 ? H[mid0].w : 0.f, p2 = on2 ? H[mid2].w : 0.f;
+    if (on0) {
+      if (p0 < phi1) lo0 = mid0 + 1; else hi0 = mid0;
+    }
+    if (on2) {
+      if (p2 < phi1) lo2 = mid2 + 1; else hi2 = mid2;
+    }
   }
-  a = lo - 1 >= f ? lo - 1 : lo;
-  b = lo < l ? lo : lo - 1;
+  c0[0] = lo0 - 1 >= f0 ? lo0 - 1 : lo0;
+  c0[1] = lo0 < l0 ? lo0 : lo0 - 1;
+  c2[0] = lo2 - 1 >= f2 ? lo2 - 1 : lo2;
+  c2[1] = lo2 < l2 ? lo2 : lo2 - 1;
 }
 
 // Twelve features of h1 (module m) with windows [f0, l0) in module m+2 and [f2, l2) in
@@ -381,12 +392,10 @@ __device__ __forceinline__ void seed_features(const float4* H, const uint8_t* si
                                               int l0, int f2, int l2, float (&f)[kMlpFeatures])
 {
   const float4 p1 = H[h1];
-  int a0, b0, a2, b2;
-  bracket(H, f0, l0, p1.w, a0, b0);
-  bracket(H, f2, l2, p1.w, a2, b2);
-  const int c0[2] = {a0, b0}, c2[2] = {a2, b2};
+  int c0[2], c2[2];
+  bracket_pair(H, f0, l0, f2, l2, p1.w, c0, c2);
   float best = 3.402823466e+38f;
-  int h0 = a0, h2 = a2;
+  int h0 = c0[0], h2 = c2[0];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
