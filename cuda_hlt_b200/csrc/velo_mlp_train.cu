@@ -339,19 +339,37 @@ struct AdamArgs {
   float* loss_total;  // += sum of the step's CTA losses
 };
 
-// Sums the per-CTA gradients in CTA order, applies one Adam step to the trainable slots
-// and publishes the bf16 copies (row-major and the two transposed blocks).
-__global__ void mlp_adam_kernel(AdamArgs A)
+// Sums the per-CTA gradients in a fixed order, applies one Adam step to the trainable slots
+// and publishes the bf16 copies (row-major and the two transposed blocks). A block takes 32
+// slots, each of its warps an eighth of the CTAs: bound by the latency of the partial sums'
+// loads, of which a thread that takes all 128 in turn keeps too few in flight (10.7 us a
+// step of 128 CTAs).
+constexpr uint32_t kAdamWarps = 8;
+static_assert(kMlpParams % 32 == 0, "a block takes 32 whole slots");
+
+__global__ void __launch_bounds__(32 * kAdamWarps) mlp_adam_kernel(AdamArgs A)
 {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p == 0 && A.loss_total) {
-    float l = 0.f;
-    for (uint32_t c = 0; c < A.parts; ++c) l += A.loss[c];
-    *A.loss_total += l;
-  }
-  if (p >= kMlpParams) return;
+  __shared__ float s_g[kAdamWarps][32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t p = blockIdx.x * 32 + lane;
+  const uint32_t per = (A.parts + kAdamWarps - 1) / kAdamWarps;
+  const uint32_t lo = min(A.parts, warp * per), hi = min(A.parts, lo + per);
   float g = 0.f;
-  for (uint32_t c = 0; c < A.parts; ++c) g += A.partial[static_cast<size_t>(c) * kMlpParams + p];
+#pragma unroll 8
+  for (uint32_t c = lo; c < hi; ++c) g += A.partial[static_cast<size_t>(c) * kMlpParams + p];
+  s_g[warp][lane] = g;
+  __syncthreads();
+  if (warp == 1 && blockIdx.x == 0 && A.loss_total) {
+    float l = 0.f;
+    for (uint32_t c = lane; c < A.parts; c += 32) l += A.loss[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
+    if (lane == 0) *A.loss_total += l;
+  }
+  if (warp != 0) return;
+  g = 0.f;
+#pragma unroll
+  for (uint32_t w = 0; w < kAdamWarps; ++w) g += s_g[w][lane];
   if (A.grad_out) A.grad_out[p] = g;
   float w = A.master[p];
   if (A.update && trainable(p)) {
@@ -596,7 +614,7 @@ int publish(VeloMlpTrainer* t, uint32_t parts, float* grad, int update, float lr
   a.grad_out = grad;
   a.loss = t->d_loss;
   a.loss_total = parts ? t->d_loss_total : nullptr;
-  mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, t->stream>>>(a);
+  mlp_adam_kernel<<<kMlpParams / 32, 32 * kAdamWarps, 0, t->stream>>>(a);
   TCK(cudaGetLastError());
   return 0;
 }
