@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <vector>
 
@@ -524,6 +525,10 @@ struct VeloMlpTrainer {
   __nv_bfloat16 *d_w = nullptr, *d_w2t = nullptr, *d_w3t = nullptr;
   float *d_partial = nullptr, *d_loss = nullptr, *d_loss_total = nullptr, *d_grad = nullptr;
   uint32_t* d_error = nullptr;
+  // rows and logits of velo_mlp_infer, kept between calls up to kKeptRows rows
+  float *d_rows = nullptr, *d_logits = nullptr;
+  uint32_t rows_cap = 0;
+  std::mutex rows_mutex;  // one call at a time uses them
   uint8_t* d_hit_labels = nullptr;
   size_t hit_labels_cap = 0;
   uint32_t grid = 0;
@@ -552,7 +557,8 @@ cudaError_t talloc(T*& p, size_t count)
 void trainer_free(VeloMlpTrainer* t)
 {
   void* ptrs[] = {t->d_feat, t->d_lab, t->d_perm, t->d_master, t->d_m, t->d_v, t->d_norm, t->d_w, t->d_w2t, t->d_w3t,
-                  t->d_partial, t->d_loss, t->d_loss_total, t->d_grad, t->d_error, t->d_hit_labels};
+                  t->d_partial, t->d_loss, t->d_loss_total, t->d_grad, t->d_error, t->d_hit_labels, t->d_rows,
+                  t->d_logits};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (t->stream) cudaStreamDestroy(t->stream);
@@ -918,9 +924,29 @@ int velo_mlp_infer(VeloMlpTrainer* t, const float* features, uint32_t n, float* 
 {
   if (!t || !features || !logits || n == 0) return VELO_ERR_INVALID;
   if (cudaSetDevice(t->device) != cudaSuccess) return VELO_ERR_CUDA;
-  float *d_f = nullptr, *d_z = nullptr;
-  TCK(talloc(d_f, 12ull * n));
-  TCK(talloc(d_z, 2ull * n));
+  // up to kKeptRows rows (56 MB) go through buffers that stay with the trainer: allocating and
+  // freeing them took half of a call on 100,000 rows
+  constexpr uint32_t kKeptRows = 1u << 20;
+  std::lock_guard<std::mutex> lock(t->rows_mutex);
+  float *d_f = t->d_rows, *d_z = t->d_logits;
+  if (n > kKeptRows) {
+    d_f = d_z = nullptr;
+    TCK(talloc(d_f, 12ull * n));
+    const cudaError_t e = talloc(d_z, 2ull * n);
+    if (e != cudaSuccess) cudaFree(d_f);
+    TCK(e);
+  } else if (n > t->rows_cap) {
+    if (t->d_rows) cudaFree(t->d_rows);
+    if (t->d_logits) cudaFree(t->d_logits);
+    t->d_rows = t->d_logits = nullptr;
+    t->rows_cap = 0;
+    const uint32_t cap = std::min(kKeptRows, std::max(n + n / 4, 4096u));
+    TCK(talloc(t->d_rows, 12ull * cap));
+    TCK(talloc(t->d_logits, 2ull * cap));
+    t->rows_cap = cap;
+    d_f = t->d_rows;
+    d_z = t->d_logits;
+  }
   TCK(cudaMemcpyAsync(d_f, features, 48ull * n, cudaMemcpyHostToDevice, t->stream));
   MlpDevice m{};
   m.w = t->d_w;
@@ -931,8 +957,10 @@ int velo_mlp_infer(VeloMlpTrainer* t, const float* features, uint32_t n, float* 
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) TCK(cudaMemcpyAsync(logits, d_z, 8ull * n, cudaMemcpyDeviceToHost, t->stream));
   TCK(cudaStreamSynchronize(t->stream));
-  cudaFree(d_f);
-  cudaFree(d_z);
+  if (n > kKeptRows) {
+    cudaFree(d_f);
+    cudaFree(d_z);
+  }
   TCK(le);
   return check_error(t);
 }
