@@ -145,6 +145,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
 __device__ __forceinline__ void load_canon(uint8_t* dst, const __nv_bfloat16* src, uint32_t rows, uint32_t k)
 {
   const uint32_t kbs = k / 8, sbo = kbs * 128u;
+#pragma unroll 4
   for (uint32_t c = threadIdx.x; c < rows * kbs; c += blockDim.x) {
     const uint32_t row = c / kbs, kb = c % kbs;
     const uint4 v = *reinterpret_cast<const uint4*>(src + row * k + kb * 8);
