@@ -12,7 +12,7 @@ namespace velo {
 // of when it runs.
 //
 // It also says how many of the first events take a block instead of a warp (queue[5]): those
-// above the caller's cluster count, and those whose search on one warp would last longer than
+// above the caller's cluster count or what a warp's search holds, and those whose search on one warp would last longer than
 // kBlockShare of a warp's share of the batch, by an estimate of a search's time, n (n + 2000)
 // for n clusters. Search in ms at shares 0.5 / 0.75 / 1 / 1.4: 4,001 events at nu ~ U(2,15)
 // 0.92 / 0.94 / 0.91 / 1.03, 8,191 at U(2,20) 1.47 / 1.41 / 1.32 / 1.29, 16,384 3.47 / 3.30 /
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kOrderThreads) order_events_kernel(ChainPointe
   const float mid = static_cast<float>(clusters) + 0.5f * (1u << kOrderShift);
   const float cost = mid * (mid + 2000.f);
   const float all = order_sum(v * cost, s_sum);
-  const bool block = clusters + (1u << kOrderShift) - 1u > P.block_threshold ||
+  const bool block = clusters + (1u << kOrderShift) - 1u > min(P.block_threshold, kWarpHitCap) ||
                      cost * static_cast<float>(P.search_warps) > kBlockShare * all;
   const float n_block = order_sum(block ? static_cast<float>(v) : 0.f, s_sum);
   if (t == 0) P.queue[5] = static_cast<uint32_t>(n_block);

@@ -353,14 +353,15 @@ union SeedArea<G, true> {
   };
 };
 
-// Shared state of one event searched by G warps.
-template<int G>
+// Shared state of one event of at most kHits hits searched by G warps.
+template<int G, uint32_t kHits = kEventHitCap>
 struct SearchShared {
+  static constexpr int kWarps = G;
   static constexpr uint32_t kFwdStage = SeedArea<G>::kFwdStage;
   SeedArea<G> u;
-  uint32_t used[kEventHitCap / 32];
-  uint32_t mstart[kModules];
-  uint32_t mnum[kModules];
+  uint32_t used[kHits / 32];
+  uint16_t mstart[kModules];
+  uint16_t mnum[kModules];
   uint32_t count[2][G];  // counts of the warps (group_rank), two in turn
   uint32_t sum;          // OR of the flags and sum of the track hits at the end
   uint32_t flags;
@@ -392,10 +393,11 @@ __device__ __forceinline__ void group_sync()
 // Exclusive rank of each thread over the group for three predicates (each count <= 32 G fits 10
 // bits), and the totals. `turn` alternates between two count buffers, so one barrier a call
 // suffices: a buffer is written again only after the barrier of the call between.
-template<int G>
-__device__ __forceinline__ void group_rank(SearchShared<G>& sh, uint32_t& turn, bool p0, bool p1, bool p2,
+template<class Shared>
+__device__ __forceinline__ void group_rank(Shared& sh, uint32_t& turn, bool p0, bool p1, bool p2,
                                            uint32_t (&rank)[3], uint32_t (&total)[3])
 {
+  constexpr int G = Shared::kWarps;
   const uint32_t lt = (1u << lane_id()) - 1u;
   const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, p0), b1 = __ballot_sync(0xFFFFFFFFu, p1),
                  b2 = __ballot_sync(0xFFFFFFFFu, p2);
@@ -524,8 +526,8 @@ struct StoredWindows {
 // (FillCandidates.cu:31-68): h0 window in module m + 2, h2 window in module m - 2.
 struct ComputedWindows {
   const float4* H;
-  const uint32_t* mstart;
-  const uint32_t* mnum;
+  const uint16_t* mstart;
+  const uint16_t* mnum;
   __device__ __forceinline__ uint2 operator()(uint32_t h1, uint32_t m) const
   {
     const float p = H[h1].w;
@@ -539,15 +541,16 @@ struct ComputedWindows {
 
 // Loads the module table of one event into the group's shared state and clears its used-hit
 // bitmask. module_start holds absolute hit indices; base is the event's first hit.
-template<int G>
-__device__ __forceinline__ void search_event_setup(SearchShared<G>& sh, const uint32_t* module_start,
+template<class Shared>
+__device__ __forceinline__ void search_event_setup(Shared& sh, const uint32_t* module_start,
                                                    const uint32_t* module_num, uint32_t base, uint32_t nhits)
 {
+  constexpr int G = Shared::kWarps;
   const uint32_t tid = group_thread<G>();
   for (uint32_t i = tid; i < (nhits + 31) / 32; i += 32 * G) sh.used[i] = 0u;
   for (uint32_t m = tid; m < kModules; m += 32 * G) {
-    sh.mstart[m] = module_start[m] - base;
-    sh.mnum[m] = module_num[m];
+    sh.mstart[m] = static_cast<uint16_t>(module_start[m] - base);
+    sh.mnum[m] = static_cast<uint16_t>(module_num[m]);
   }
   if (tid == 0) {
     sh.sum = 0;
@@ -563,15 +566,16 @@ __device__ __forceinline__ void search_event_setup(SearchShared<G>& sh, const ui
 // number of tracks written to sc.track_n / sc.track_hits; status bits go to `flags` (per
 // thread: OR-reduce them over the group). Every append is ranked in the order of one warp
 // taking the work from the front, so the result does not depend on G.
-template<int G, class Windows>
-__device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const float4* H, const Windows& windows,
+template<class Shared, class Windows>
+__device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, const Windows& windows,
                                                  const uint8_t* KE, const EventScratch& sc, uint32_t& flags)
 {
+  constexpr int G = Shared::kWarps;
   const uint32_t lane = lane_id(), tid = group_thread<G>();
   const uint32_t warp = G == 1 ? 0u : threadIdx.x >> 5;
   uint32_t* used = sh.used;
-  const uint32_t* mstart = sh.mstart;
-  const uint32_t* mnum = sh.mnum;
+  const uint16_t* mstart = sh.mstart;
+  const uint16_t* mnum = sh.mnum;
   SeedSlots& sl = sh.u.seed[warp];
   uint16_t* track_n = sc.track_n;
   uint16_t* track_hits = sc.track_hits;
@@ -586,7 +590,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
   // seeding's first run (fetch).
   auto stage = [&](uint32_t first) {
     const uint32_t mo = first - 4, me = first - 5, mon = mnum[mo], men = mnum[me];
-    if (mon + men > SearchShared<G>::kFwdStage) return;
+    if (mon + men > Shared::kFwdStage) return;
     const float4 *Ho = H + mstart[mo], *He = H + mstart[me];
     for (uint32_t i = tid; i < mon; i += 32 * G) async_copy4(&sh.u.fphi[i], &Ho[i].w);
     for (uint32_t i = tid; i < men; i += 32 * G) async_copy4(&sh.u.fphi[mon + i], &He[i].w);
@@ -749,7 +753,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
     const float moz = c_module_z[mo], mez = c_module_z[me];
     // the phi of both target modules in shared memory, where their searches stay; a pair of
     // modules above the staging size is searched in global memory
-    const bool fits = mon + men <= SearchShared<G>::kFwdStage;
+    const bool fits = mon + men <= Shared::kFwdStage;
     const float* sphi_o = fits ? sh.u.fphi : nullptr;
     const float* sphi_e = fits ? sh.u.fphi + mon : nullptr;
     if constexpr (kFetchAhead<G>) {
@@ -806,7 +810,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
       }
       const bool is_new = action == 1 && nhit == 3;
       uint32_t rank[3], total[3];  // new tracks, tracks followed on, weak tracklets
-      group_rank<G>(sh, turn, is_new, action == 1 || action == 2, action == 3, rank, total);
+      group_rank(sh, turn, is_new, action == 1 || action == 2, action == 3, rank, total);
       // new tracks beyond the last slot are dropped, and not followed
       const uint32_t slot = n_tracks + rank[0];
       const uint32_t dropped = slot > kMaxTracks ? slot - kMaxTracks : 0u;  // before this thread's
@@ -879,7 +883,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
       if (i < diff) full = ttf[(prev + i) % kTtfModulo].x;
       const bool is_weak = i < diff && (full & 0x80000000u);
       uint32_t rank[3], total[3];
-      group_rank<G>(sh, turn, is_weak, false, false, rank, total);
+      group_rank(sh, turn, is_weak, false, false, rank, total);
       if (is_weak && weak_ptr + rank[0] < kWeakCap) {
         const uint32_t tp = full & 0x0FFFFFFFu;
         uint16_t* w = weak + 3 * (weak_ptr + rank[0]);
@@ -907,7 +911,7 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
       accept = !any_used && chi2 < kMaxChi2;
     }
     uint32_t rank[3], total[3];
-    group_rank<G>(sh, turn, accept, false, false, rank, total);
+    group_rank(sh, turn, accept, false, false, rank, total);
     if (accept) {
       const uint32_t slot = n_tracks + rank[0];
       if (slot < kMaxTracks) {
@@ -926,9 +930,10 @@ __device__ __forceinline__ uint32_t search_event(SearchShared<G>& sh, const floa
 }
 
 // One event of the chain by G warps: its tracks, their count and hit count and its status.
-template<int G>
-__device__ __forceinline__ void search_chain_event(SearchShared<G>& sh, const ChainPointers& P, uint32_t e)
+template<class Shared>
+__device__ __forceinline__ void search_chain_event(Shared& sh, const ChainPointers& P, uint32_t e)
 {
+  constexpr int G = Shared::kWarps;
   const uint32_t lane = lane_id(), tid = group_thread<G>();
   const uint32_t nhits = P.event_hits[e];
   const uint32_t status = P.status[e];
@@ -938,14 +943,14 @@ __device__ __forceinline__ void search_chain_event(SearchShared<G>& sh, const Ch
   const bool runnable = !(status & (kStatusBadRawEvent | kStatusHitOverflow)) && nhits <= kEventHitCap && nhits > 0;
   if (nhits > kEventHitCap) flags |= kStatusHitOverflow;
   if (runnable) {
-    search_event_setup<G>(sh, P.module_start + e * kModules, P.module_num + e * kModules, base, nhits);
+    search_event_setup(sh, P.module_start + e * kModules, P.module_num + e * kModules, base, nhits);
     const EventScratch sc{P.scratch.track_n + static_cast<size_t>(e) * kMaxTracks,
                           P.scratch.track_hits + static_cast<size_t>(e) * kMaxTracks * kMaxTrackSize,
                           P.scratch.tracklets + static_cast<size_t>(e) * kTrackletRing * 3,
                           P.scratch.ttf + static_cast<size_t>(e) * kTtfModulo,
                           P.scratch.weak + static_cast<size_t>(e) * kWeakCap * 3};
     const uint8_t* KE = (P.keep && P.mlp.use_ext) ? P.keep + base : nullptr;  // extension pruning
-    n_tracks = search_event<G>(sh, P.hits.xyzp + base, StoredWindows{P.windows + base}, KE, sc, flags);
+    n_tracks = search_event(sh, P.hits.xyzp + base, StoredWindows{P.windows + base}, KE, sc, flags);
     for (uint32_t t = tid; t < n_tracks; t += 32 * G) track_hits += sc.track_n[t];
   }
   flags = __reduce_or_sync(0xFFFFFFFFu, flags);
@@ -993,7 +998,7 @@ __global__ void __launch_bounds__(W * 32, 32 / W) search_kernel(ChainPointers P)
 {
   __shared__ union {
     SearchShared<W> block;
-    SearchShared<1> warp[W];
+    SearchShared<1, kWarpHitCap> warp[W];
   } s;
   __shared__ uint32_t s_next;
   const uint32_t lane = lane_id();
@@ -1005,14 +1010,14 @@ __global__ void __launch_bounds__(W * 32, 32 / W) search_kernel(ChainPointers P)
     const uint32_t q = s_next;
     __syncthreads();
     if (q >= n_block) break;
-    search_chain_event<W>(s.block, P, P.event_order[q]);
+    search_chain_event(s.block, P, P.event_order[q]);
   }
   for (;;) {
     uint32_t q = 0;
     if (lane == 0) q = n_block + atomicAdd(P.queue + 1, 1u);
     q = __shfl_sync(0xFFFFFFFFu, q, 0);
     if (q >= n_events) break;
-    search_chain_event<1>(s.warp[threadIdx.x >> 5], P, P.event_order[q]);
+    search_chain_event(s.warp[threadIdx.x >> 5], P, P.event_order[q]);
   }
 }
 

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(128) search_static_kernel(StaticSearchArgs A)
     const bool runnable = !(status & (kStatusBadRawEvent | kStatusHitOverflow)) && nhits <= kEventHitCap && nhits > 0;
     if (nhits > kEventHitCap) flags |= kStatusHitOverflow;
     if (runnable) {
-      search_event_setup<1>(sw, A.module_start + e * kModules, A.module_num + e * kModules, base, nhits);
+      search_event_setup(sw, A.module_start + e * kModules, A.module_num + e * kModules, base, nhits);
       const float4* H = A.xyzp + base;
       uint8_t* ev_scratch = A.scratch + kStaticHeaderBytes + static_cast<size_t>(e) * kEventScratchBytes;
       const EventScratch sc{A.track_n + static_cast<size_t>(e) * kMaxTracks,
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(128) search_static_kernel(StaticSearchArgs A)
                             reinterpret_cast<uint16_t*>(ev_scratch),
                             reinterpret_cast<uint2*>(ev_scratch + kTrackletBytes),
                             reinterpret_cast<uint16_t*>(ev_scratch + kTrackletBytes + kTtfBytes)};
-      n_tracks = search_event<1>(sw, H, ComputedWindows{H, sw.mstart, sw.mnum}, nullptr, sc, flags);
+      n_tracks = search_event(sw, H, ComputedWindows{H, sw.mstart, sw.mnum}, nullptr, sc, flags);
     }
     uint32_t f = flags;
 #pragma unroll
