@@ -437,17 +437,19 @@ __global__ void __launch_bounds__(W * 32) consolidate_fit_kernel(ChainPointers P
     const uint32_t carry = first_hit + chunk0;
     // coalesced write of the chunk's hit range [carry, carry + chunk_hits)
     const bool staged = chunk_hits <= kConsolidateStage;
-    // four output positions per lane at a time: their dependent gathers (hit index, then
-    // record and id) are in flight together. The track of a position: every track has hits,
+    // eight output positions per lane at a time, as many as 32 average tracks have: their dependent
+    // gathers (hit index, then record and id) are in flight together (65,536 events 1.98 ms with
+    // four, 1.78 with eight at 96 registers, 1.87 with nine at 111; four at 64 registers, which one
+    // more block an SM would need, 3.24). The track of a position: every track has hits,
     // so the tracks starting inside 32 consecutive positions are marked by one bit each (an
     // OR across the warp of the lanes' own starts) and counted with a popcount.
     const uint32_t my_start = lane < n_chunk ? s_off[i] - chunk0 : 0xFFFFFFFFu;
     uint32_t started = 0;  // tracks starting before the current group of 32 positions
-    for (uint32_t base = 0; base < chunk_hits; base += 4 * 32) {  // warp-uniform
+    for (uint32_t base = 0; base < chunk_hits; base += 8 * 32) {  // warp-uniform
       const uint32_t j0 = base + lane;
-      uint32_t hh[4];
+      uint32_t hh[8];
 #pragma unroll
-      for (uint32_t u = 0; u < 4; ++u) {
+      for (uint32_t u = 0; u < 8; ++u) {
         const uint32_t p0 = base + 32 * u;  // first position of this group
         const uint32_t heads =
           __reduce_or_sync(0xFFFFFFFFu, my_start - p0 < 32u ? 1u << (my_start - p0) : 0u);
@@ -456,17 +458,17 @@ __global__ void __launch_bounds__(W * 32) consolidate_fit_kernel(ChainPointers P
         started += __popc(heads);
         hh[u] = j < chunk_hits ? track_hits[(i0 + t) * kMaxTrackSize + (chunk0 + j - s_off[i0 + t])] : 0u;
       }
-      float4 p[4];
-      uint32_t id[4];
+      float4 p[8];
+      uint32_t id[8];
 #pragma unroll
-      for (uint32_t u = 0; u < 4; ++u) {
+      for (uint32_t u = 0; u < 8; ++u) {
         if (j0 + 32 * u < chunk_hits) {
           p[u] = H[hh[u]];
           id[u] = ids[hh[u]];
         }
       }
 #pragma unroll
-      for (uint32_t u = 0; u < 4; ++u) {
+      for (uint32_t u = 0; u < 8; ++u) {
         const uint32_t j = j0 + 32 * u;
         if (j < chunk_hits) {
           ox[carry + j] = p[u].x;
