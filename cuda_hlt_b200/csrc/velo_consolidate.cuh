@@ -15,37 +15,13 @@ __device__ __forceinline__ void store_totals(const ChainPointers& P, uint32_t tr
   P.totals[2] = P.queue[6];
 }
 
-// The scans of a batch that exceeds the consolidated output capacity, event after event: one
-// that does not fit what is left keeps no tracks, so every offset stays inside the buffers.
-__device__ __forceinline__ void scan_events_in_turn(const ChainPointers& P)
-{
-  const uint32_t N = P.run->n_events;
-  uint32_t ot = 0, oh = 0;
-  for (uint32_t e = 0; e < N; ++e) {
-    uint32_t nt = P.event_tracks[e], nh = P.event_track_hits[e];
-    if (static_cast<uint64_t>(ot) + nt > P.max_tracks_total || static_cast<uint64_t>(oh) + nh > P.max_track_hits_total) {
-      P.status[e] |= kStatusTrackOverflow;
-      nt = 0;
-      nh = 0;
-      P.event_tracks[e] = 0;
-      P.event_track_hits[e] = 0;
-    }
-    P.atomics[e] = nt;
-    P.atomics[N + e] = ot;
-    P.event_hit_offset[e] = oh;
-    ot += nt;
-    oh += nh;
-  }
-  P.atomics[2 * N] = ot;
-  P.event_hit_offset[N] = oh;
-  P.track_hit_number[ot] = oh;
-  store_totals(P, ot, oh);
-}
-
 // Exclusive scans of tracks and track hits per event by one block of 1024 threads, in the
 // layout of copy_and_prefix_sum_single_block + the track-hit prefix sum
-// (PrefixSumSingleBlock.cu:130-168).
-__global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
+// (PrefixSumSingleBlock.cu:130-168). An event beyond the consolidated output capacity keeps no
+// tracks: each thread drops those of its run of events that do not fit behind the sum of all
+// events before the run, so the totals of such a batch may lie beyond the capacity; nothing is
+// written there.
+__device__ __forceinline__ void scan_events_one_block(const ChainPointers& P)
 {
   __shared__ uint32_t s_warp_t[32], s_warp_h[32];
   const uint32_t N = P.run->n_events;
@@ -85,14 +61,19 @@ __global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
     s_warp_h[lane] = wh;
   }
   __syncthreads();
-  if (s_warp_t[31] > P.max_tracks_total || s_warp_h[31] > P.max_track_hits_total) {
-    if (threadIdx.x == 0) scan_events_in_turn(P);
-    return;
-  }
   uint32_t ot = it - t + (warp ? s_warp_t[warp - 1] : 0);
   uint32_t oh = ih - h + (warp ? s_warp_h[warp - 1] : 0);
   for (uint32_t e = a; e < b; ++e) {
-    const uint32_t nt = P.event_tracks[e], nh = P.event_track_hits[e];
+    uint32_t nt = P.event_tracks[e];
+    uint32_t nh = P.event_track_hits[e];
+    if (ot + nt > P.max_tracks_total || oh + nh > P.max_track_hits_total) {
+      // consolidated output capacity exhausted: the event keeps no tracks
+      P.status[e] |= kStatusTrackOverflow;
+      nt = 0;
+      nh = 0;
+      P.event_tracks[e] = 0;
+      P.event_track_hits[e] = 0;
+    }
     P.atomics[e] = nt;
     P.atomics[N + e] = ot;
     P.event_hit_offset[e] = oh;
@@ -103,15 +84,20 @@ __global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
   if (b == N && (a < b || (N == 0 && threadIdx.x == 0))) {
     P.atomics[2 * N] = ot;
     P.event_hit_offset[N] = oh;
-    P.track_hit_number[ot] = oh;
+    if (ot <= P.max_tracks_total) P.track_hit_number[ot] = oh;
     store_totals(P, ot, oh);
   }
+}
+
+__global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
+{
+  scan_events_one_block(P);
 }
 
 // The same scans for batches of more than kScanOneBlock events, kScanBlock events a block in two
 // launches: one block walks a thread's run of events one after the other, at uncoalesced
 // addresses, and takes 4.8 us per 1,000 events (65,536: 0.315 ms, so 0.014). A batch that exceeds
-// the output capacity is scanned in turn.
+// the output capacity goes through the one block, whose rule for what is dropped holds then.
 constexpr uint32_t kScanBlock = 1024;
 constexpr uint32_t kScanOneBlock = 4096;
 
@@ -162,7 +148,7 @@ __global__ void __launch_bounds__(kScanBlock) event_scan_blocks_kernel(ChainPoin
   }
   const ulonglong2 all = scan_block_sum(at, ah, s_sum), before = scan_block_sum(bt, bh, s_sum);
   if (all.x > P.max_tracks_total || all.y > P.max_track_hits_total) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) scan_events_in_turn(P);
+    if (blockIdx.x == 0) scan_events_one_block(P);
     return;
   }
   const uint32_t e = blockIdx.x * kScanBlock + threadIdx.x;
@@ -393,6 +379,8 @@ __global__ void __launch_bounds__(W * 32) consolidate_fit_kernel(ChainPointers P
   const uint32_t Htot = P.event_hit_offset[N];
   const uint32_t nt = P.atomics[e];
   if (nt == 0) return;
+  // the totals of a batch beyond the output capacity may not fit the buffers they lay out
+  if (49ull * T > 52ull * P.max_tracks_total || Htot > P.max_track_hits_total) return;
   const uint32_t t0 = P.atomics[N + e];
   const float4* H = P.hits.xyzp + P.event_hit_base[e];
   const uint32_t* ids = P.hits.id + P.event_hit_base[e];

@@ -303,8 +303,8 @@ int velo_run_gec_host(VeloCtx* ctx, const void* raw_host, const uint64_t* raw_of
                       const VeloGecInput* gec_host, uint32_t n_events, void* stream, VeloOutputs* out);
 
 /* Waits for the context's last run (its stream); fills totals (tracks, track hits, clusters).
- * The track and track-hit totals are read into pinned memory at the end of every run, so the
- * wait does not queue behind copies issued on the stream's copy engine since. */
+ * Every run writes the track and track-hit totals to pinned memory, so the wait does not queue
+ * behind copies issued on the stream's copy engine since. */
 int velo_sync(VeloCtx* ctx, uint32_t* total_tracks, uint32_t* total_track_hits, uint64_t* total_clusters);
 
 /* ---- learned seed/extension scorer (no counterpart in the reference) ----

@@ -103,28 +103,32 @@ def test_module_sizes_at_the_edges_of_the_sorts(geometry, copies):
 
 
 @pytest.mark.parametrize("n", [4096, 4097, 5121])
-@pytest.mark.parametrize("capacity", [1.0, 0.4])
+@pytest.mark.parametrize("capacity", [1.0, 0.97])
 def test_event_scan_and_output_capacity(n, capacity):
     """Above 4,096 events the scan runs over many blocks. In a batch beyond the output capacity
-    an event that does not fit what is left of it keeps no tracks and is flagged."""
+    the rule of the one-block scan holds: 1,024 runs of events, each from the sum of all events
+    before it, an event that does not fit keeps no tracks and is flagged."""
     b = events.generate(n, seed=9, nu_min=0.6, nu_max=0.6, with_mc=False)
     full, (T, H, _) = run(b)
     assert T > 2 * n
-    nt, hits = full["n_tracks"].astype(np.int64), np.diff(full["track_hit_number"].astype(np.int64))
-    nh = np.add.reduceat(np.append(hits, 0), np.minimum(full["track_offsets"][:-1], T)) * (nt > 0)
-    assert np.array_equal(full["track_offsets"], np.concatenate([[0], np.cumsum(nt)])) and nh.sum() == H
+    nt = full["n_tracks"].astype(np.int64)
+    starts = np.concatenate([[0], np.cumsum(nt)])
+    assert np.array_equal(full["track_offsets"], starts) and full["track_hit_number"][T] == H
     cap_t = int(T * capacity)
-    res, totals = run(b, max_tracks=cap_t, max_track_hits=16 * T)
-    kept, over, at = np.zeros(n, np.int64), np.zeros(n, bool), 0
-    for e in range(n):
-        over[e] = at + nt[e] > cap_t
-        kept[e] = 0 if over[e] else nt[e]
-        at += kept[e]
-    want = np.concatenate([[0], np.cumsum(kept)])
-    assert np.array_equal(res["n_tracks"], kept)
-    assert np.array_equal(res["track_offsets"], want) and totals[0] == want[n]
-    # the events that stay are whole
-    for e in np.flatnonzero(kept)[::97]:
-        assert event_bits(res, e) == event_bits(full, e), e
-    dropped = (res["status"] & chain.STATUS["track_overflow"]) != 0
-    assert np.array_equal(dropped, over) and over.any() == (capacity < 1)
+    vc = chain.VeloChain(max_events=n, max_raw_bytes=int(b.raw.size) + 4096, max_tracks=cap_t, max_track_hits=16 * T)
+    vc.run_host(b)
+    totals = vc.sync()
+    atomics, status = (vc._down(p, np.uint32, k) for p, k in ((vc.out.atomics, 2 * n + 1), (vc.out.status, n)))
+    vc.close()
+    per = -(-n // 1024)
+    kept, over, offsets = np.zeros(n, np.int64), np.zeros(n, bool), np.zeros(n + 1, np.int64)
+    for a in range(0, n, per):
+        at = starts[a]
+        for e in range(a, min(n, a + per)):
+            over[e] = at + nt[e] > cap_t
+            kept[e] = 0 if over[e] else nt[e]
+            offsets[e] = at
+            at += kept[e]
+        offsets[n] = at
+    assert np.array_equal(atomics[:n], kept) and np.array_equal(atomics[n:], offsets) and totals[0] == offsets[n]
+    assert np.array_equal((status & chain.STATUS["track_overflow"]) != 0, over) and over.any() == (capacity < 1)
