@@ -17,26 +17,31 @@ __device__ __forceinline__ void store_totals(const ChainPointers& P, uint32_t tr
 
 // Exclusive scans of tracks and track hits per event by one block of 1024 threads, in the
 // layout of copy_and_prefix_sum_single_block + the track-hit prefix sum
-// (PrefixSumSingleBlock.cu:130-168). An event beyond the consolidated output capacity keeps no
-// tracks: each thread drops those of its run of events that do not fit behind the sum of all
-// events before the run, so the totals of such a batch may lie beyond the capacity; nothing is
-// written there.
+// (PrefixSumSingleBlock.cu:130-168). Sum holds the tracks and track hits of the whole batch.
+//
+// An event beyond the consolidated output capacity keeps no tracks and is flagged: each thread
+// drops those of its run of events that do not fit behind the sum of all events before the run.
+// So one run, where the sums pass the capacity, may keep some of its events, the runs before it
+// keep all and those behind it none. The offsets and the totals count the kept events only:
+// what is kept lies packed inside the buffers, and all of it is written.
+template<class Sum>
 __device__ __forceinline__ void scan_events_one_block(const ChainPointers& P)
 {
-  __shared__ uint32_t s_warp_t[32], s_warp_h[32];
+  __shared__ Sum s_warp_t[32], s_warp_h[32];
+  __shared__ uint32_t s_kept_t, s_kept_h;  // of a batch beyond the capacity
   const uint32_t N = P.run->n_events;
   const uint32_t per = (N + blockDim.x - 1) / blockDim.x;
   const uint32_t a = min(N, threadIdx.x * per), b = min(N, a + per);
-  uint32_t t = 0, h = 0;
+  Sum t = 0, h = 0;
   for (uint32_t e = a; e < b; ++e) {
     t += P.event_tracks[e];
     h += P.event_track_hits[e];
   }
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  uint32_t it = t, ih = h;
+  Sum it = t, ih = h;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t vt = __shfl_up_sync(0xFFFFFFFFu, it, o), vh = __shfl_up_sync(0xFFFFFFFFu, ih, o);
+    const Sum vt = __shfl_up_sync(0xFFFFFFFFu, it, o), vh = __shfl_up_sync(0xFFFFFFFFu, ih, o);
     if (lane >= static_cast<uint32_t>(o)) {
       it += vt;
       ih += vh;
@@ -48,10 +53,10 @@ __device__ __forceinline__ void scan_events_one_block(const ChainPointers& P)
   }
   __syncthreads();
   if (warp == 0) {
-    uint32_t wt = lane < (blockDim.x >> 5) ? s_warp_t[lane] : 0, wh = lane < (blockDim.x >> 5) ? s_warp_h[lane] : 0;
+    Sum wt = lane < (blockDim.x >> 5) ? s_warp_t[lane] : 0, wh = lane < (blockDim.x >> 5) ? s_warp_h[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t vt = __shfl_up_sync(0xFFFFFFFFu, wt, o), vh = __shfl_up_sync(0xFFFFFFFFu, wh, o);
+      const Sum vt = __shfl_up_sync(0xFFFFFFFFu, wt, o), vh = __shfl_up_sync(0xFFFFFFFFu, wh, o);
       if (lane >= static_cast<uint32_t>(o)) {
         wt += vt;
         wh += vh;
@@ -61,37 +66,55 @@ __device__ __forceinline__ void scan_events_one_block(const ChainPointers& P)
     s_warp_h[lane] = wh;
   }
   __syncthreads();
-  uint32_t ot = it - t + (warp ? s_warp_t[warp - 1] : 0);
-  uint32_t oh = ih - h + (warp ? s_warp_h[warp - 1] : 0);
-  for (uint32_t e = a; e < b; ++e) {
-    uint32_t nt = P.event_tracks[e];
-    uint32_t nh = P.event_track_hits[e];
-    if (ot + nt > P.max_tracks_total || oh + nh > P.max_track_hits_total) {
-      // consolidated output capacity exhausted: the event keeps no tracks
-      P.status[e] |= kStatusTrackOverflow;
-      nt = 0;
-      nh = 0;
-      P.event_tracks[e] = 0;
-      P.event_track_hits[e] = 0;
-    }
+  const Sum first_t = it - t + (warp ? s_warp_t[warp - 1] : 0), first_h = ih - h + (warp ? s_warp_h[warp - 1] : 0);
+  const bool behind = first_t > P.max_tracks_total || first_h > P.max_track_hits_total;
+  const bool over = first_t + t > P.max_tracks_total || first_h + h > P.max_track_hits_total;
+  uint32_t ot = static_cast<uint32_t>(first_t), oh = static_cast<uint32_t>(first_h);
+  auto put = [&](uint32_t e, uint32_t nt) {
     P.atomics[e] = nt;
     P.atomics[N + e] = ot;
     P.event_hit_offset[e] = oh;
-    ot += nt;
-    oh += nh;
+  };
+  auto drop = [&](uint32_t e) {
+    P.status[e] |= kStatusTrackOverflow;
+    P.event_tracks[e] = 0;
+    P.event_track_hits[e] = 0;
+    put(e, 0);
+  };
+  if (!behind) {
+    for (uint32_t e = a; e < b; ++e) {
+      const uint32_t nt = P.event_tracks[e], nh = P.event_track_hits[e];
+      if (over && (static_cast<Sum>(ot) + nt > P.max_tracks_total || static_cast<Sum>(oh) + nh > P.max_track_hits_total)) {
+        drop(e);
+        continue;
+      }
+      put(e, nt);
+      ot += nt;
+      oh += nh;
+    }
+    if (over) {  // one thread: every later run starts behind the capacity
+      s_kept_t = ot;
+      s_kept_h = oh;
+    }
+  }
+  if (__syncthreads_or(behind) && behind) {
+    ot = s_kept_t;
+    oh = s_kept_h;
+    for (uint32_t e = a; e < b; ++e) drop(e);
   }
   // the last thread that owns events (or thread 0 when N == 0) writes the totals
   if (b == N && (a < b || (N == 0 && threadIdx.x == 0))) {
     P.atomics[2 * N] = ot;
     P.event_hit_offset[N] = oh;
-    if (ot <= P.max_tracks_total) P.track_hit_number[ot] = oh;
+    P.track_hit_number[ot] = oh;
     store_totals(P, ot, oh);
   }
 }
 
+// (one block takes at most kScanOneBlock events: their sums fit 32 bits)
 __global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
 {
-  scan_events_one_block(P);
+  scan_events_one_block<uint32_t>(P);
 }
 
 // The same scans for batches of more than kScanOneBlock events, kScanBlock events a block in two
@@ -100,6 +123,7 @@ __global__ void __launch_bounds__(1024) event_scan_kernel(ChainPointers P)
 // the output capacity goes through the one block, whose rule for what is dropped holds then.
 constexpr uint32_t kScanBlock = 1024;
 constexpr uint32_t kScanOneBlock = 4096;
+static_assert(static_cast<uint64_t>(kScanOneBlock) * kMaxTracks * kMaxTrackSize < (1ull << 32), "32-bit sums");
 
 // Sum over the block of x and y; s_sum: 32 entries.
 __device__ __forceinline__ ulonglong2 scan_block_sum(unsigned long long x, unsigned long long y, ulonglong2* s_sum)
@@ -148,7 +172,7 @@ __global__ void __launch_bounds__(kScanBlock) event_scan_blocks_kernel(ChainPoin
   }
   const ulonglong2 all = scan_block_sum(at, ah, s_sum), before = scan_block_sum(bt, bh, s_sum);
   if (all.x > P.max_tracks_total || all.y > P.max_track_hits_total) {
-    if (blockIdx.x == 0) scan_events_one_block(P);
+    if (blockIdx.x == 0) scan_events_one_block<unsigned long long>(P);
     return;
   }
   const uint32_t e = blockIdx.x * kScanBlock + threadIdx.x;
@@ -379,8 +403,6 @@ __global__ void __launch_bounds__(W * 32) consolidate_fit_kernel(ChainPointers P
   const uint32_t Htot = P.event_hit_offset[N];
   const uint32_t nt = P.atomics[e];
   if (nt == 0) return;
-  // the totals of a batch beyond the output capacity may not fit the buffers they lay out
-  if (49ull * T > 52ull * P.max_tracks_total || Htot > P.max_track_hits_total) return;
   const uint32_t t0 = P.atomics[N + e];
   const float4* H = P.hits.xyzp + P.event_hit_base[e];
   const uint32_t* ids = P.hits.id + P.event_hit_base[e];

@@ -129,8 +129,7 @@ __global__ void __launch_bounds__(kPvThreads) pv_beamline_kernel(ChainPointers P
   const uint32_t e = P.event_order[blockIdx.x];  // largest first
   const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
   const uint32_t T = P.atomics[2 * N];
-  // (no states stand behind totals that lie beyond the output capacity)
-  const uint32_t nt = 49ull * T > 52ull * P.max_tracks_total ? 0u : P.atomics[e];
+  const uint32_t nt = P.atomics[e];
   const uint32_t t0 = P.atomics[N + e];
   const float* K = reinterpret_cast<const float*>(V.kalman);
   PvTrack* tracks = V.tracks + t0;

@@ -21,16 +21,27 @@ def run(b, max_tracks=0, max_track_hits=0, **kw):
     return res, totals
 
 
-def event_bits(res, e):
-    """Everything the chain says of one event, as comparable bytes."""
+def bits(parts):
+    return b"".join(np.ascontiguousarray(p).tobytes() for p in parts)
+
+
+def track_bits(res, e):
+    """The tracks of one event, their states and, behind the vertex stage, its vertices."""
     t0, t1 = int(res["track_offsets"][e]), int(res["track_offsets"][e + 1])
     h0, h1 = int(res["track_hit_number"][t0]), int(res["track_hit_number"][t1])
     parts = [res["status"][e], res["track_hit_number"][t0:t1 + 1] - h0, res["hit_id"][h0:h1]]
     parts += [res[k][h0:h1] for k in ("hit_x", "hit_y", "hit_z")]
-    parts += [res[s][k][t0:t1] for s in ("states", "kalman") for k in chain.STATE_FIELDS]
-    for m in chain.event_clusters(res, e):
-        parts += [m[k] for k in ("id", "phi", "x", "y", "z", "size")]
-    return b"".join(np.ascontiguousarray(p).tobytes() for p in parts)
+    parts += [res[s][k][t0:t1] for s in ("states", "kalman") for k in chain.STATE_FIELDS + ("backward",)]
+    if "pv_count" in res:
+        parts += [res["pv_count"][e], res["pv_vertices"][e, :res["pv_count"][e]], res["pv_npeaks"][e],
+                  res["pv_zpeaks"][e, :res["pv_npeaks"][e]]]
+    return bits(parts)
+
+
+def event_bits(res, e):
+    """Everything the chain says of one event, as comparable bytes."""
+    parts = [m[k] for m in chain.event_clusters(res, e) for k in ("id", "phi", "x", "y", "z", "size")]
+    return track_bits(res, e) + bits(parts)
 
 
 @pytest.fixture(scope="module")
@@ -102,33 +113,68 @@ def test_module_sizes_at_the_edges_of_the_sorts(geometry, copies):
     assert event_bits(res, 0) == event_bits(res, b.n_events - 2)
 
 
-@pytest.mark.parametrize("n", [4096, 4097, 5121])
-@pytest.mark.parametrize("capacity", [1.0, 0.97])
-def test_event_scan_and_output_capacity(n, capacity):
-    """Above 4,096 events the scan runs over many blocks. In a batch beyond the output capacity
-    the rule of the one-block scan holds: 1,024 runs of events, each from the sum of all events
-    before it, an event that does not fit keeps no tracks and is flagged."""
-    b = events.generate(n, seed=9, nu_min=0.6, nu_max=0.6, with_mc=False)
-    full, (T, H, _) = run(b)
-    assert T > 2 * n
-    nt = full["n_tracks"].astype(np.int64)
-    starts = np.concatenate([[0], np.cumsum(nt)])
-    assert np.array_equal(full["track_offsets"], starts) and full["track_hit_number"][T] == H
-    cap_t = int(T * capacity)
-    vc = chain.VeloChain(max_events=n, max_raw_bytes=int(b.raw.size) + 4096, max_tracks=cap_t, max_track_hits=16 * T)
+@pytest.fixture(scope="module")
+def full_run():
+    """Batches of n events, their results with the vertex stage and nothing left out, and their
+    events as bytes."""
+    cache = {}
+
+    def get(n):
+        if n not in cache:
+            b = events.generate(n, seed=9, nu_min=0.6, nu_max=0.6, with_mc=False)
+            vc = chain.VeloChain(max_events=n, max_raw_bytes=int(b.raw.size) + 4096)
+            vc.set_pv(True)
+            vc.run_host(b)
+            T, H, _ = vc.sync()
+            res = vc.results()
+            vc.close()
+            assert T > 2 * n and H == res["track_hit_number"][T]
+            assert np.array_equal(res["track_offsets"], np.concatenate([[0], np.cumsum(res["n_tracks"])]))
+            res["n_hits"] = np.diff(res["track_hit_number"][res["track_offsets"]].astype(np.int64))
+            cache[n] = b, res, T, H, [track_bits(res, e) for e in range(n)]
+        return cache[n]
+    return get
+
+
+# 4,096 events and less are scanned by one block, more by many
+@pytest.mark.parametrize("n", [5, 1025, 4096, 4097, 5121])
+@pytest.mark.parametrize("tracks, hits", [(1.0, 1.0), (0.97, 1.0), (0.4, 1.0), (1.0, 0.97), (1.0, 0.4), (0.4, 0.97)])
+@pytest.mark.parametrize("pv", [False, True])
+def test_event_scan_and_output_capacity(full_run, n, tracks, hits, pv):
+    """Of a batch beyond the output capacity every event is that of the full run, byte for byte,
+    or flagged and without tracks, whatever an earlier run left in the buffers. The rule of the
+    scan: 1,024 runs of events, each from the sum of all events before it; an event that does not
+    fit keeps no tracks; what is kept lies packed."""
+    b, full, T, H, want = full_run(n)
+    cap_t, cap_h = int(T * tracks), int(H * hits)
+    vc = chain.VeloChain(max_events=n, max_raw_bytes=2 * int(b.raw.size) + 4096, max_tracks=cap_t, max_track_hits=cap_h)
+    vc.set_pv(pv)
+    vc.run_host(events.generate(n, seed=10, nu_min=0.9, nu_max=0.9, with_mc=False))
+    vc.sync()
     vc.run_host(b)
     totals = vc.sync()
-    atomics, status = (vc._down(p, np.uint32, k) for p, k in ((vc.out.atomics, 2 * n + 1), (vc.out.status, n)))
+    res = vc.results()
     vc.close()
+
+    nt, nh = full["n_tracks"].astype(np.int64), full["n_hits"]
+    st, sh = (np.concatenate([[0], np.cumsum(v)]) for v in (nt, nh))
     per = -(-n // 1024)
-    kept, over, offsets = np.zeros(n, np.int64), np.zeros(n, bool), np.zeros(n + 1, np.int64)
+    over = np.zeros(n, bool)
     for a in range(0, n, per):
-        at = starts[a]
+        t, h = st[a], sh[a]
         for e in range(a, min(n, a + per)):
-            over[e] = at + nt[e] > cap_t
-            kept[e] = 0 if over[e] else nt[e]
-            offsets[e] = at
-            at += kept[e]
-        offsets[n] = at
-    assert np.array_equal(atomics[:n], kept) and np.array_equal(atomics[n:], offsets) and totals[0] == offsets[n]
-    assert np.array_equal((status & chain.STATUS["track_overflow"]) != 0, over) and over.any() == (capacity < 1)
+            over[e] = t + nt[e] > cap_t or h + nh[e] > cap_h
+            t, h = (t, h) if over[e] else (t + nt[e], h + nh[e])
+    assert over.any() == (tracks < 1 or hits < 1) and not over.all()
+    kept = np.where(over, 0, nt)
+    assert np.array_equal(res["n_tracks"], kept)
+    assert np.array_equal(res["track_offsets"], np.concatenate([[0], np.cumsum(kept)]))
+    assert totals[:2] == (kept.sum(), np.where(over, 0, nh).sum()) and totals[0] <= cap_t and totals[1] <= cap_h
+    assert np.array_equal((res["status"] & chain.STATUS["track_overflow"]) != 0, over)
+    if not pv:
+        full = {k: v for k, v in full.items() if not k.startswith("pv_")}
+        want = [track_bits(full, e) for e in range(n)]
+    for e in range(n):
+        assert track_bits(res, e) == want[e] or over[e], e
+    if pv:
+        assert not res["pv_count"][over].any()
