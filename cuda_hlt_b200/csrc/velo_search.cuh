@@ -585,6 +585,11 @@ __device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, co
   uint32_t n_tracks = 0, tracklet_ptr = 0, ttf_ptr = 0, weak_ptr = 0;
   uint32_t last_seeded = 0;
   uint32_t turn = 0;
+  // An event with more tracks to follow than the ring holds overwrites entries before they are
+  // read, and may follow a track twice: what becomes of it depends on how many entries are read
+  // ahead of the writes. From the first step that can come to that (kStatusTtfOverflow follows
+  // if it does), one warp takes 32 entries in turn, as G = 1 does.
+  bool in_turn = false;
 
   // Ahead of their step: the phi of the forwarding's modules (stage) and the windows of the
   // seeding's first run (fetch).
@@ -763,8 +768,14 @@ __device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, co
       for (uint32_t i = tid; i < men; i += 32 * G) sh.u.fphi[mon + i] = H[mes + i].w;
     }
     group_sync<G>();
-    for (uint32_t i0 = 0; i0 < diff; i0 += 32 * G) {
-      const uint32_t i = i0 + tid;
+    uint32_t step = 32 * G;
+    for (uint32_t i0 = 0; i0 < diff; i0 += step) {
+      if constexpr (G > 1) {
+        // from here on the ring's writes may pass its reads
+        if (ttf_ptr + 32 * G > prev_ttf + i0 + kTtfModulo) in_turn = true;
+        if (in_turn) step = 32;
+      }
+      const uint32_t i = tid < step ? i0 + tid : diff;
       int action = 0;  // 1 extend, 2 keep with a skipped module, 3 demote to weak
       uint32_t full = 0, last_two = 0, trackno = 0, nhit = 0;
       uint16_t t0 = 0, best_h2 = 0;
@@ -848,6 +859,7 @@ __device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, co
         w[2] = static_cast<uint16_t>(last_two >> 16);
       }
       weak_ptr += total[2];
+      if (G == 1 || in_turn) group_sync<G>();
     }
     group_sync<G>();
   };

@@ -178,3 +178,63 @@ def test_event_scan_and_output_capacity(full_run, n, tracks, hits, pv):
         assert track_bits(res, e) == want[e] or over[e], e
     if pv:
         assert not res["pv_count"][over].any()
+
+
+def tiled(b, n):
+    """n copies of a batch, one after the other."""
+    size = int(b.offsets[-1])
+    off = np.concatenate([b.offsets[:-1] + np.uint64(k * size) for k in range(n)] + [[np.uint64(n * size)]])
+    return events.EventBatch(np.tile(b.raw, n), off.astype(np.uint64))
+
+
+def overfull_event(rng, modules):
+    """125 clusters a sensor over the same 64 x 64 SPs of each: everything near everything, so that
+    more tracks are followed than the ring holds."""
+    payload, offs = [], [0]
+    for sensor in range(208):
+        n = 125 if sensor // 4 in modules else 0
+        a = np.sort(rng.choice(64 * 64, n, replace=False))
+        payload += [sensor, n] + [0x80000000 | ((int(x) // 64) << 6 | int(x) % 64) << 8 | 1 << int(rng.integers(8)) for x in a]
+        offs.append(4 * len(payload))
+    return np.array([208] + offs + payload, np.uint32).view(np.uint8)
+
+
+def test_ring_overflow_does_not_depend_on_the_batch():
+    """Events that overflow the ring of tracks to follow, which the reference leaves undefined: the
+    same tracks on one warp, on four and on eight, whatever the batch."""
+    import torch
+    rng = np.random.default_rng(1)
+    few = [overfull_event(rng, range(a, a + k)) for a, k in ((10, 8), (25, 8), (38, 14))]
+    off = np.concatenate([[0], np.cumsum([e.size for e in few])]).astype(np.uint64)
+    b = events.EventBatch(np.concatenate(few), off)
+    # eight warps an event
+    vc = chain.VeloChain(max_events=3, max_raw_bytes=int(b.raw.size) + 4096, max_tracks=3600)
+    vc.run_host(b)
+    vc.sync()
+    res = vc.results()
+    assert np.all(res["status"] & chain.STATUS["ttf_overflow"]) and res["n_tracks"].min() > 100
+    want = [track_bits(res, e) for e in range(3)]
+    # one warp an event, windows computed in place
+    track_n, track_hits = (torch.zeros(3 * 1200 * k, dtype=torch.int16, device="cuda") for k in (1, 26))
+    n_tracks, status = (torch.zeros(3, dtype=torch.int32, device="cuda") for _ in range(2))
+    status_in = torch.from_numpy(res["status"].astype(np.int32) & chain.STATUS["candidate_overflow"]).cuda()
+    o = vc.out
+    assert vc.lib.velo_search_static(o.hit_xyzp, o.module_hit_start, o.module_hit_num, status_in.data_ptr(), 3,
+                                     track_n.data_ptr(), track_hits.data_ptr(), n_tracks.data_ptr(), status.data_ptr(),
+                                     torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    vc.close()
+    assert np.array_equal(n_tracks.cpu().numpy(), res["n_tracks"]) and np.array_equal(status.cpu().numpy(), res["status"])
+    tn, th = track_n.cpu().numpy().reshape(3, 1200), track_hits.cpu().numpy().view(np.uint16).reshape(3, 1200, 26)
+    for e in range(3):
+        ids = res["cluster_id"][int(res["module_start"][52 * e]):]
+        assert [tuple(ids[th[e, t, :tn[e, t]]]) for t in range(n_tracks[e])] == chain.event_tracks(res, e)
+    # four warps an event, each event a large one of its batch
+    small = events.generate(700, seed=3, nu_min=2.0, nu_max=4.0, with_mc=False)
+    mixed = events.EventBatch(np.concatenate([b.raw, small.raw]), np.concatenate([b.offsets, small.offsets[1:] + b.offsets[3]]))
+    got, _ = run(mixed)
+    assert [track_bits(got, e) for e in range(3)] == want
+    # one warp an event in a full device (the third, the larger one, takes a block)
+    n = 1600
+    got, _ = run(tiled(b, n), max_tracks=1200 * 3 * n)
+    assert all(track_bits(got, e) == want[e % 3] for e in range(3 * n))
