@@ -663,6 +663,7 @@ static int launch_run(VeloCtx* c, const void* raw, const uint64_t* raw_offsets, 
     VCK(cudaMemsetAsync(c->d_atomics, 0, sizeof(uint32_t), s));
     VCK(cudaMemsetAsync(c->d_track_hit_number, 0, sizeof(uint32_t), s));
     VCK(cudaMemsetAsync(c->d_event_hit_offset, 0, sizeof(uint32_t), s));
+    VCK(cudaMemsetAsync(c->d_queue, 0, 8 * sizeof(uint32_t), s));  // as set_run_kernel does
     if (gec) VCK(cudaMemsetAsync(c->d_n_selected, 0, sizeof(uint32_t), s));
     return 0;
   }

@@ -242,6 +242,23 @@ def test_edge_cases_empty_corrupt_and_ragged(geometry):
     vc.close()
 
 
+def test_empty_batch_reports_no_earlier_error():
+    """An empty batch is a run of its own: neither what a destroyed context left in the device
+    memory nor an earlier run's timeout is its error."""
+    empty = events.EventBatch(np.zeros(0, np.uint8), np.zeros(1, np.uint64))
+    others = []
+    for _ in range(8):  # (the others keep the memory that the contexts share alive)
+        vc, other = (chain.VeloChain(max_events=4, max_raw_bytes=1 << 16) for _ in range(2))
+        others.append(other)
+        for _ in range(2):
+            vc.run_host(empty)
+            assert vc.sync() == (0, 0, 0)
+            assert vc.lib.velo_check_wait_timeout(vc.ctx, 4096, None) == 0  # sets the error word
+        vc.close()
+    for other in others:
+        other.close()
+
+
 def test_capacity_errors():
     b = events.generate_config("plain_1k", n_events=8)
     vc = chain.VeloChain(max_events=4, max_raw_bytes=int(b.raw.size))
