@@ -10,9 +10,12 @@ vertices agree to 2e-3 mm in position and 1e-2 relative in chi2 and covariance (
 reference has NaN: a singular fit matrix), their track counts exactly. The float32 CPU oracle (no fused multiply-adds, libm exp) is held to the same
 bounds. Runs are bit-for-bit reproducible.
 """
+import os
+
 import numpy as np
 import pytest
 
+import oracle
 from cuda_hlt_b200 import chain, events
 
 pytestmark = pytest.mark.gpu
@@ -65,6 +68,7 @@ def compare_vertices(got, n_got, want, n_want, what):
     return differ
 
 
+@pytest.mark.skipif(not os.path.exists(oracle.REF_GPU_LIB), reason="reference GPU build missing")
 @pytest.mark.parametrize("name", ["minbias", "nu7.6", "nu2-20"])
 def test_pv_matches_reference_kernels(name):
     b = dict(batches())[name]
