@@ -291,7 +291,8 @@ def test_full_size_batch_properties():
 
 @pytest.mark.parametrize("mapping", [chain.MAP_WARP, chain.MAP_BLOCK])
 def test_search_mappings_bit_exact(mapping):
-    """Warp-per-event and block-per-event searches give the reference's result each."""
+    """The search gives the reference's result under each mapping. (In a batch this small a block
+    searches most events under either; one warp an event: test_gpu_sizes.py.)"""
     g = load_golden("batched")
     b = golden_batch("batched")
     res = run_chain(b, mapping=mapping)

@@ -5,8 +5,9 @@ import numpy as np
 import pytest
 
 import oracle
-from cuda_hlt_b200 import chain, events
-from test_gpu_windows import windows_of
+from cuda_hlt_b200 import chain, events, mlp, train_scorer
+from conftest import golden_batch
+from test_gpu_windows import PHI_CAP, windows_of
 
 pytestmark = pytest.mark.gpu
 
@@ -65,19 +66,6 @@ def test_events_do_not_depend_on_the_batch_size(batch_700, per_sm, more):
         assert event_bits(res, e) == want[e], e
 
 
-def test_large_events_search_their_windows_by_parity():
-    """More events than the wide decode takes, some above the 8,192 clusters whose phi fit the
-    shared memory together."""
-    b = events.generate_config("high_occupancy_200k", n_events=330, first_event=0, with_mc=False)
-    vc = chain.VeloChain(max_events=330, max_raw_bytes=int(b.raw.size) + 4096)
-    vc.run_host(b)
-    vc.sync()
-    res = vc.results()
-    assert res["module_num"].reshape(-1, 52).sum(1).max() > 8192
-    windows_of(vc, res, 330)
-    vc.close()
-
-
 def sp_event(rng, counts):
     """A raw event with counts[m] isolated one-pixel SPs in module m, in address order."""
     payload, offs = [], [0]
@@ -89,6 +77,29 @@ def sp_event(rng, counts):
         payload += [sensor, n] + words
         offs.append(4 * len(payload))
     return np.array([208] + offs + payload, np.uint32).view(np.uint8)
+
+
+# blocks of 4 warps hold 6,144 phi, of 8 warps (more events than the wide decode takes) 8,192
+@pytest.mark.parametrize("copies, warps", [(2, 4), (330, 8)])
+@pytest.mark.parametrize("large", [0, 1])
+def test_modules_of_a_parity_beyond_the_shared_phi(copies, warps, large):
+    """The windows of an event whose modules of one parity hold more phi than the block's shared
+    memory: they are searched in the cluster records, the other parity's as ever."""
+    rng = np.random.default_rng(11)
+    counts = np.where(np.arange(52) % 2 == large, PHI_CAP[warps] // 26 + 5, 60)
+    ev = sp_event(rng, counts)
+    b = events.EventBatch(np.tile(ev, copies), np.arange(copies + 1, dtype=np.uint64) * np.uint64(ev.size))
+    vc = chain.VeloChain(max_events=copies, max_raw_bytes=int(b.raw.size) + 4096, max_tracks=1200 * copies,
+                         decode_warps=warps)
+    vc.run_host(b)
+    vc.sync()
+    res = vc.results()
+    assert np.array_equal(res["module_num"][:52], counts)
+    per_parity = res["module_num"][:52].reshape(26, 2).sum(0)
+    assert per_parity[large] > PHI_CAP[warps] > per_parity[1 - large] and per_parity.sum() <= 16384
+    windows_of(vc, res, 2)
+    vc.close()
+    assert event_bits(res, 0) == event_bits(res, copies - 1)
 
 
 @pytest.mark.parametrize("copies", [1, 330])
@@ -238,3 +249,67 @@ def test_ring_overflow_does_not_depend_on_the_batch():
     n = 1600
     got, _ = run(tiled(b, n), max_tracks=1200 * 3 * n)
     assert all(track_bits(got, e) == want[e % 3] for e in range(3 * n))
+
+
+def warp_events(hits, sms):
+    """Events that the order kernel's rule leaves a warp each: up to 12,288 clusters, and no longer
+    than a warp's share of the batch."""
+    mid = (np.asarray(hits, np.int64) // 16) * 16 + 8.0
+    cost = mid * (mid + 2000.0)
+    return (np.asarray(hits) < 12288) & (cost * (32 * sms) <= cost.sum())
+
+
+@pytest.mark.parametrize("mode", ["plain", "extension"])
+def test_one_warp_an_event_in_a_full_device(mode, batch_700):
+    """A batch that fills the device: most events take a warp each, the largest a block, and every
+    copy equals the event in a small batch of one block an event, whose tracks other tests compare
+    with the reference's. In the pruned mode every candidate is scored and forwarding is pruned too."""
+    sms = batch_700[2]
+    b = golden_batch("batched")
+    w = None
+    if mode == "extension":
+        w = mlp.load_weights(train_scorer.DEFAULT_WEIGHTS)
+        w.min_pairs = w.min_event_clusters = 0
+        w.ext_threshold = 0.3
+    small, full = [], []
+    for batch, mapping, out in ((b, chain.MAP_BLOCK, small), (tiled(b, 280), chain.MAP_WARP, full)):
+        vc = chain.VeloChain(max_events=batch.n_events, max_raw_bytes=int(batch.raw.size) + 4096, mapping=mapping)
+        if w is not None:
+            vc.set_mlp(w)
+            vc.set_mode(chain.MODE_PRUNED)
+        vc.run_host(batch)
+        vc.sync()
+        res = vc.results()
+        vc.close()
+        out += [track_bits(res, e) for e in range(batch.n_events)]
+    warp = warp_events(res["module_num"].reshape(-1, 52).sum(1), sms)
+    assert warp.sum() > 4000 and (~warp).sum() > 500
+    if w is not None:
+        assert not (res["status"] & chain.STATUS["mlp_fallback"]).any() and (res["cluster_keep"] & 2 == 0).any()
+    for e, got in enumerate(full):
+        assert got == small[e % 32], e
+
+
+def test_largest_events_of_one_warp():
+    """A warp's used-hit bits hold 12,288 clusters: events of 12,272 to 12,287 take one in a batch
+    that fills the device, those above a block, and each equals itself in a small batch."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(7)
+    sizes = [12272, 12286, 12287, 12288, 12289, 12304]
+    few = [sp_event(rng, np.full(52, n // 52) + (np.arange(52) < n % 52)) for n in sizes]
+    off = np.concatenate([[0], np.cumsum([e.size for e in few])]).astype(np.uint64)
+    b = events.EventBatch(np.concatenate(few), off)
+    ref, _ = run(b, max_tracks=1200 * 6)
+    assert ref["module_num"].reshape(-1, 52).sum(1).tolist() == sizes and ref["n_tracks"].min() > 0
+    want = [track_bits(ref, e) for e in range(6)]
+    n = 6 * (7 * 32 * sms // 36)
+    assert warp_events(sizes * (n // 6), sms).tolist() == [True, True, True, False, False, False] * (n // 6)
+    many = tiled(b, n // 6)
+    vc = chain.VeloChain(max_events=n, max_raw_bytes=int(many.raw.size) + 4096, max_tracks=1200 * n, max_track_hits=6000 * n)
+    vc.run_host(many)
+    vc.sync()
+    res = vc.results(clusters=False)
+    vc.close()
+    for e in range(n):
+        assert track_bits(res, e) == want[e % 6], e

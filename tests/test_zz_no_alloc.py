@@ -1,5 +1,5 @@
-"""velo_search_static, the search entry point that allocates nothing, against the chain's
-own warp-per-event search on the same clusters.
+"""velo_search_static, the search entry point that allocates nothing (one warp an event),
+against the chain's own search of the same clusters.
 
 Some callers cannot allocate device memory: a host framework that reserves the whole device
 at start-up and hands its plugins fixed slices of that reservation (as the stage this
@@ -42,7 +42,7 @@ def _static_tracks(cluster_id, module_start, track_n, track_hits, event_tracks, 
 def test_static_search_matches_chain(config, n, first):
     import torch
     b = events.generate_config(config, n_events=n, first_event=first)
-    # the chain's warp-per-event search is the one the entry point shares its code with
+    # (in a batch of this size a block of eight warps searches most events)
     vc = chain.VeloChain(max_events=n, max_raw_bytes=int(b.raw.size) + 4096, mapping=chain.MAP_WARP)
     vc.run_host(b)
     vc.sync()
