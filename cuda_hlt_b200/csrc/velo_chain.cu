@@ -76,7 +76,7 @@ struct VeloCtx {
   uint32_t* d_queue = nullptr;
   uint32_t* d_event_order = nullptr;
   ulonglong2* d_scan_sums = nullptr;
-  uint32_t block_threshold = 0;  // clusters above which an event takes the block search
+  uint32_t block_threshold = 0;  // clusters above which an event takes a block in the search
   // beamline PV stage (velo_set_pv)
   bool pv = false;
   PvTrack* d_pv_tracks = nullptr;
@@ -112,7 +112,6 @@ struct VeloCtx {
   uint32_t ev_next = 0;
   int ev_current = -1;
   int decode_warps = 8;
-  int search_wpb = 4;
   uint32_t decode_blocks = 0, search_blocks = 0, fill_blocks = 0,
            feature_blocks = 0, score_blocks = 0;
   // CUDA graphs per (batch-size bucket, stream, global event cut on or off): the kernels read
@@ -934,7 +933,7 @@ int velo_sync(VeloCtx* c, uint32_t* total_tracks, uint32_t* total_track_hits, ui
   if (cudaSetDevice(c->device) != cudaSuccess) return VELO_ERR_CUDA;
   cudaStream_t s = c->last_stream;
   const uint32_t N = c->last_n;
-  VCK(cudaStreamSynchronize(s));  // the totals were queued behind the run
+  VCK(cudaStreamSynchronize(s));  // the run wrote the totals
   if (c->h_totals[2]) return VELO_ERR_DEVICE_TIMEOUT;
   if (total_tracks) *total_tracks = c->h_totals[0];
   if (total_track_hits) *total_track_hits = c->h_totals[1];

@@ -154,8 +154,8 @@ struct ChainPointers {
   uint32_t max_tracks_total;
   uint32_t max_track_hits_total;
   uint64_t hit_capacity;       // entries of the hit SoA arrays
-  // work queues: [0] decode, [1] warp search, [2] block search, [5] events of the block
-  // search, [6] error bits, [7] candidate rows
+  // work queues: [0] decode, [1] search, events that take a warp, [2] search, events that take a
+  // block, [5] how many take a block, [6] error bits, [7] candidate rows
   uint32_t* queue;             // [8]
   uint32_t* event_order;       // [N] events, largest first: the search's queue order
   uint32_t block_threshold;    // events with more clusters than this take a block in the search
@@ -240,8 +240,8 @@ __device__ __forceinline__ uint32_t orderable(float f)
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-// phi-window searches of cuda/velo/common/include/VeloTools.cuh:6-42 (the "found" flag
-// accumulates over every probed element, as there).
+// The phi-window searches of cuda/velo/common/include/VeloTools.cuh:6-42 (the "found" flag
+// accumulates over every probed element, as there): the first one over phi in shared memory.
 __device__ __forceinline__ int window_first(const float* a, uint32_t size, float value, float margin)
 {
   bool found = false;
@@ -255,16 +255,7 @@ __device__ __forceinline__ int window_first(const float* a, uint32_t size, float
   found |= fabsf(value - a[l]) < margin;
   return found ? l : -1;
 }
-__device__ __forceinline__ int window_second(const float* a, uint32_t size, float value, float margin)
-{
-  int l = 0, r = static_cast<int>(size) - 1;
-  while (l < r) {
-    const int m = (l + r) / 2;
-    if (value + margin > a[m]) l = m + 1; else r = m;
-  }
-  return fabsf(value - a[l]) < margin ? l + 1 : l;
-}
-// The same two searches over the phi lane (.w) of the float4 cluster records.
+// Both searches over the phi lane (.w) of the float4 cluster records.
 __device__ __forceinline__ int window_first4(const float4* a, uint32_t size, float value, float margin)
 {
   bool found = false;
@@ -287,6 +278,7 @@ __device__ __forceinline__ int window_second4(const float4* a, uint32_t size, fl
   }
   return fabsf(value - a[l].w) < margin ? l + 1 : l;
 }
+// [first, last) of the hits of a phi-sorted module within margin of value; first = -1 if none.
 __device__ __forceinline__ void phi_window4(const float4* H, uint32_t start, uint32_t num, float value, float margin,
                                             int& first, int& last)
 {
@@ -299,20 +291,7 @@ __device__ __forceinline__ void phi_window4(const float4* H, uint32_t start, uin
   }
 }
 
-// [first, last) of hits in a phi-sorted module within margin of value; first = -1 if none.
-__device__ __forceinline__ void phi_window(const float* phis, uint32_t start, uint32_t num, float value, float margin,
-                                           int& first, int& last)
-{
-  first = window_first(phis + start, num, value, margin);
-  last = -1;
-  if (first != -1) {
-    const int s = window_second(phis + start + first, num - first, value, margin);
-    first += start;
-    last = s == 0 ? first + 1 : first + s;
-  }
-}
-
-// phi_window over n (> 0) sorted phi in shared memory, n the same for every lane of the warp:
+// phi_window4 over n (> 0) sorted phi in shared memory, n the same for every lane of the warp:
 // the partition points of the reference's two searches by halving steps without a branch, and
 // its "found" flag from the elements beside the first one. The flag says whether an element
 // that the search probes lies within the margin. The one it ends on is probed; when that one

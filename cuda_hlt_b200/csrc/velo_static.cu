@@ -52,7 +52,7 @@ struct StaticSearchArgs {
 };
 
 // Warp per event, events pulled from the counter at the head of the scratch. The search of
-// each event is the chain's warp search (search_event_warp, velo_search.cuh), with its seeding
+// each event is the chain's by one warp (search_event, velo_search.cuh), with its seeding
 // windows computed in place instead of read from fill_candidates' output.
 __global__ void __launch_bounds__(128) search_static_kernel(StaticSearchArgs A)
 {
