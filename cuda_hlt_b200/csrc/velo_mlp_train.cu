@@ -145,6 +145,10 @@ __global__ void __launch_bounds__(kMlpTile, 1) mlp_train_kernel(TrainArgs A)
   const uint32_t t = threadIdx.x;
   if (t < 32) tmem_alloc(&s.tmem, kTrainTmemCols);
   if (t == 0) mbar_init1(&s.mbar);
+  // A successor may start from here on: it must not take the tensor memory that a CTA of this
+  // step has yet to allocate. One training CTA fills an SM's shared memory, so a successor's
+  // waits for this one's end; were two to fit, launch_next would belong behind the allocation.
+  static_assert(2 * kTrainSmem > 227 * 1024, "one training CTA an SM");
   launch_next();
   if (t < 32) s.norm[t] = A.norm[t];
   // rows of the transposed operands that no sample writes stay zero

@@ -56,7 +56,10 @@ extern "C" {
 #define VELO_STATUS_MODULE_OVERFLOW (1u << 1)
 #define VELO_STATUS_HIT_OVERFLOW (1u << 2)
 #define VELO_STATUS_CANDIDATE_OVERFLOW (1u << 3)
-#define VELO_STATUS_TRACK_OVERFLOW (1u << 4)
+#define VELO_STATUS_TRACK_OVERFLOW (1u << 4) /* more than 1,200 tracks (the first 1,200 are kept), or
+                                                beyond VeloConfig.max_tracks / max_track_hits, where the
+                                                event keeps none: the other events' outputs and the
+                                                totals lie inside the buffers */
 #define VELO_STATUS_TTF_OVERFLOW (1u << 5)
 #define VELO_STATUS_WEAK_OVERFLOW (1u << 6)
 #define VELO_STATUS_H1_OVERFLOW (1u << 7)
@@ -158,13 +161,15 @@ typedef struct VeloCtx VeloCtx;
                               (velo_capture_labels): a perfect scorer at no cost, which measures
                               how much pruning can save at most */
 
-/* Search mapping. A warp searches an event, or a block of four warps does: the events above the
- * boundary of velo_set_block_threshold, and those whose search on one warp would outlast a
- * warp's share of the batch (a batch too small to fill the device gives every event a
- * block). The tracks do not depend on it. */
+/* Search mapping. A warp searches an event, or a block does: the events above the boundary of
+ * velo_set_block_threshold, those above 12,288 clusters, and those whose search on one warp would
+ * outlast a warp's share of the batch (in a batch too small to fill the device all but the
+ * smallest). A block has four warps, or eight where the batch is at most four events per SM. The
+ * tracks do not depend on it, save for events with more than 512 clusters in a module
+ * (VELO_STATUS_MODULE_OVERFLOW), whose cluster order is not defined. */
 #define VELO_MAP_AUTO 0    /* search: no boundary */
 #define VELO_MAP_BLOCK 1   /* search: one block per event */
-#define VELO_MAP_WARP 2    /* search: no boundary */
+#define VELO_MAP_WARP 2    /* the same as VELO_MAP_AUTO, kept for the programs that name it */
 
 typedef struct VeloConfig {
   uint32_t max_events;          /* events per velo_run call */
@@ -398,13 +403,15 @@ int velo_download_async(VeloCtx* ctx, void* dst_host, const void* src_device, si
  * default. */
 int velo_set_pv(VeloCtx* ctx, int enabled);
 
-/* Search mapping: events with more than `clusters` clusters always take a block in the search
- * (0: all, >= 16384: none but those the mapping's own rule gives one). Set by the autotuner
+/* Search mapping: events with more than `clusters` clusters (compared in steps of 16) always
+ * take a block in the search (0: all, >= 16384: none but those the mapping's own rule gives
+ * one). Set by the autotuner
  * (cuda_hlt_b200/autotune.py) from timings per hit-count bucket. */
 int velo_set_block_threshold(VeloCtx* ctx, uint32_t clusters);
 
 /* Decode block size: 4 or 8 warps per event (default 8, of which a batch of at most two events
- * per SM makes 16); set by the autotuner (cuda_hlt_b200/autotune.py) from decode timings on a
+ * per SM makes 16; with CUDA graphs the size of the batch's bucket counts here and for the
+ * search's blocks); set by the autotuner (cuda_hlt_b200/autotune.py) from decode timings on a
  * sample batch. */
 int velo_set_decode_warps(VeloCtx* ctx, uint32_t warps);
 
