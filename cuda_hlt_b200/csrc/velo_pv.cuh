@@ -121,7 +121,10 @@ struct PvSmem {
   uint32_t vkeep[kPvMaxVertices];
 };
 
-__global__ void __launch_bounds__(kPvThreads) pv_beamline_kernel(ChainPointers P, PvPointers V)
+// 9 blocks per SM: left to itself the compiler takes 48 registers for 10, which costs the fits
+// more than the tenth block gives (4,096 events at nu ~ U(2,20) 0.304 ms, so, with 55, 0.287;
+// 8 blocks 0.296).
+__global__ void __launch_bounds__(kPvThreads, 9) pv_beamline_kernel(ChainPointers P, PvPointers V)
 {
   __shared__ PvSmem s;
   const uint32_t N = P.run->n_events;
