@@ -559,7 +559,7 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
   uint8_t pat[256], sizes[256];
   float fx[512], fy[512];
   velo_build_sp_luts(pat, sizes, fx, fy);
-  std::vector<SpCluster> sp(512);
+  std::array<SpCluster, 512> sp;  // (no allocation here that could throw through the C entry)
   for (int m = 0; m < 256; ++m)
     for (int k = 0; k < 2; ++k) {
       const uint32_t row = k ? (pat[m] >> 4) & 3u : pat[m] & 3u, col = k ? (pat[m] >> 6) & 1u : (pat[m] >> 2) & 1u;
@@ -567,9 +567,9 @@ int velo_create(const VeloConfig* cfg, const void* geometry, size_t geometry_byt
       sp[2 * m + k] = SpCluster{fx[2 * m + k], fy[2 * m + k],
                                 row | col << 2 | more | static_cast<uint32_t>((sizes[m] >> (4 * k)) & 0xF) << 4, 0u};
     }
-  std::vector<float> blob(kGeometryBytes / 4);  // the caller's may stand at any address
+  std::array<float, kGeometryBytes / 4> blob;  // the caller's may stand at any address
   std::memcpy(blob.data(), geometry, kGeometryBytes);
-  std::vector<float2> column(kPixelColumns);
+  std::array<float2, kPixelColumns> column;
   for (uint32_t i = 0; i < kPixelColumns; ++i) column[i] = make_float2(blob[i], blob[kSensorColumns + i]);
   if (cudaMemcpy(c->d_ltg, blob.data() + 2 * kSensorColumns, kSensors * 64, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(c->d_local_x, column.data(), column.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
