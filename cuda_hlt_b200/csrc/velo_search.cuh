@@ -768,13 +768,10 @@ __device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, co
       for (uint32_t i = tid; i < men; i += 32 * G) sh.u.fphi[mon + i] = H[mes + i].w;
     }
     group_sync<G>();
-    uint32_t step = 32 * G;
+    // the writes come nearest to the reads at the start: an entry read writes at most one
+    in_turn |= diff + 32 * G > kTtfModulo;
+    const uint32_t step = in_turn ? 32 : 32 * G;
     for (uint32_t i0 = 0; i0 < diff; i0 += step) {
-      if constexpr (G > 1) {
-        // from here on the ring's writes may pass its reads
-        if (ttf_ptr + 32 * G > prev_ttf + i0 + kTtfModulo) in_turn = true;
-        if (in_turn) step = 32;
-      }
       const uint32_t i = tid < step ? i0 + tid : diff;
       int action = 0;  // 1 extend, 2 keep with a skipped module, 3 demote to weak
       uint32_t full = 0, last_two = 0, trackno = 0, nhit = 0;
@@ -859,7 +856,7 @@ __device__ __forceinline__ uint32_t search_event(Shared& sh, const float4* H, co
         w[2] = static_cast<uint16_t>(last_two >> 16);
       }
       weak_ptr += total[2];
-      if (G == 1 || in_turn) group_sync<G>();
+      if (step == 32) group_sync<G>();
     }
     group_sync<G>();
   };
